@@ -1046,7 +1046,7 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
   fft_group<T, LOG2N, R, -1>(W, bufX, j, tw);
   __syncthreads();
 #pragma unroll
-  for (int m = 0; m < R; ++m) bufX[spad<R, T>(j + m * G)] = W[m];
+  for (int m = 0; m < R; ++m) bufX[j + m * G] = W[m];
   __syncthreads();
   // split: Ja(kx) = (W(kx) + conj W(-kx))/2, Jb(kx) = -i (W(kx) - conj W(-kx))/2
   C* jh = reinterpret_cast<C*>(a.jh);
@@ -1056,8 +1056,8 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     const int kx = idx >> lnp;
     const int q = idx & (np - 1);
     const C* w = smem + (size_t)q * qs;
-    const C wk = w[spad<R, T>(kx)];
-    const C wm = w[spad<R, T>((N - kx) & (N - 1))];
+    const C wk = w[kx];
+    const C wm = w[(N - kx) & (N - 1)];
     const C ja = mkc<C>((T)0.5 * (wk.x + wm.x), (T)0.5 * (wk.y - wm.y));
     const C d = mkc<C>(wk.x - wm.x, wk.y + wm.y);
     const C jb = mkc<C>((T)0.5 * d.y, (T)-0.5 * d.x);
@@ -1075,7 +1075,7 @@ template <typename T, int LOG2N>
 __device__ void ring_reduce(const KP& kp, const ColArgs& a) {
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N;
-  __shared__ double red[1024];
+  __shared__ double red[256];  // V lanes
   __shared__ double s_scale;
   const int n = kp.n_ring;
   const int s = a.stage;
