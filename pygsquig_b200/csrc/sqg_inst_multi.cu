@@ -38,16 +38,26 @@ struct MultiShape {
 template <typename T, int L>
 __device__ __forceinline__ void row_multi_body(const KP& kp, const RowArgs& a, int tile) {
   using S = MultiShape<T, L>;
-  row_body<T, L, S::R, S::RPC, S::DEPTH, S::NFX>(kp, a, tile);
+  if (a.rmode == RM_P1) {
+    if (a.fmode == FM_THETA) row_body<T, L, S::R, S::RPC, S::DEPTH, S::NFX, RI_THETA_P1, true>(kp, a, tile);
+    else row_body<T, L, S::R, S::RPC, S::DEPTH, S::NFX, RI_SCAL_P1, true>(kp, a, tile);
+  } else {
+    if (a.fmode == FM_THETA) row_body<T, L, S::R, S::RPC, S::DEPTH, S::NFX, RI_THETA_STAGE, true>(kp, a, tile);
+    else row_body<T, L, S::R, S::RPC, S::DEPTH, S::NFX, RI_SCAL_STAGE, true>(kp, a, tile);
+  }
 }
 template <typename T, int L>
 __device__ __forceinline__ void col_multi_body(const KP& kp, const ColArgs& a, int tile, int ntiles) {
   using S = MultiShape<T, L>;
-  col_body<T, L, S::CR, S::NP, S::NBUF>(kp, a, tile, ntiles);
+  switch (a.cmode) {
+    case CM_THETA: col_body<T, L, S::CR, S::NP, S::NBUF, CM_THETA>(kp, a, tile, ntiles); break;
+    case CM_SCAL: col_body<T, L, S::CR, S::NP, S::NBUF, CM_SCAL>(kp, a, tile, ntiles); break;
+    default: col_body<T, L, S::CR, S::NP, S::NBUF, CM_SCALV>(kp, a, tile, ntiles); break;
+  }
 }
 
 template <typename T>
-constexpr int kMultiRowMinBlocks = 65536 / (kMultiRowThreads * (sizeof(T) == 4 ? 64 : 128));
+constexpr int kMultiRowMinBlocks = 65536 / (kMultiRowThreads * (sizeof(T) == 4 ? 72 : 128));
 template <typename T>
 __global__ void __launch_bounds__(kMultiRowThreads, kMultiRowMinBlocks<T>)
 k_row_multi(const MultiArgs ma) {

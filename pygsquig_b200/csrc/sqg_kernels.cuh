@@ -24,6 +24,8 @@
 // (k, -k) reproduces the reference exactly, including at the Nyquist row and
 // column where a derivative multiplier is not Hermitian-symmetric.
 #pragma once
+#include <type_traits>
+
 #include "pdl.cuh"
 #include "sqg_fft.cuh"
 #include "sqg_tma.cuh"
@@ -42,29 +44,46 @@ struct RowTab {
   int dmax, dragmax, pos_lo, pos_hi, neg_lo, neg_hi, row_start, pad;
 };
 
+// The band of a field: the disk p <= pmax, p^2 + m_y^2 <= s2 (mode numbers) that
+// holds the dealiasing mask.  Modes outside it -- half of a spectrum's rows
+// times columns, a third of the rows p = 0..N/2 entirely -- get no advective
+// tendency, so a spectrum that is zero there stays zero through a step, and a
+// run's is: what an initial field holds there decays by hyperviscosity alone,
+// and a spectrum interpolated or restarted from a band-limited one never held
+// any.  The input pass of a step sets one byte per row pair, tl[p] = 1 when the
+// pair holds a non-zero mode outside the band.  With tl[p] = 0 the stage passes
+// load, update and store the band's modes only, and a row beyond pmax costs
+// its block one byte: no transforms, no half-spectrum rows (the column pass
+// takes unwritten rows as zero).  Rows with tl[p] = 1 take every mode, as they
+// do when tl is null.  Independent of tl, the transformed Jacobian is neither
+// written nor read nor transformed beyond pmax, where the mask discards it.
 enum FieldMode { FM_THETA = 0, FM_VEL = 1, FM_PHYS1 = 2, FM_SCAL = 3 };
 enum RowMode { RM_P1 = 0, RM_STAGE = 1, RM_RHS = 2, RM_SPEC = 3 };
-// Row-pass instances: one that reads its modes from the arguments; the stage
-// passes of theta and of the scalars compiled for their modes alone (any
-// stage), or for their modes and one stage s = 1..4 (RI_THETA_S1 + s - 1,
-// RI_SCAL_S1 + s - 1); the input passes (RM_P1) of theta, of the scalars and
-// of the velocity.
+// Row-pass instances: one that reads its modes from the arguments (the batch
+// passes), and instances compiled for their modes alone: the stage passes of
+// theta and of the scalars (any stage, or one stage s = 1..4, RI_THETA_S1 + s -
+// 1, RI_SCAL_S1 + s - 1); the input passes (RM_P1) of theta, of the scalars, of
+// the velocity and of a plain field; the right-hand side; the forward
+// transform.
 enum RowInst {
   RI_ANY = 0, RI_THETA_STAGE = 1, RI_SCAL_STAGE = 2, RI_THETA_S1 = 3, RI_SCAL_S1 = 7,
-  RI_THETA_P1 = 11, RI_SCAL_P1 = 12, RI_VEL_P1 = 13
+  RI_THETA_P1 = 11, RI_SCAL_P1 = 12, RI_VEL_P1 = 13, RI_PHYS_P1 = 14, RI_RHS = 15, RI_SPEC = 16
 };
 __host__ __device__ constexpr int ri_fmode(int ri) {
-  return (ri == RI_THETA_STAGE || ri == RI_THETA_P1 || (ri >= RI_THETA_S1 && ri < RI_SCAL_S1)) ? FM_THETA
+  return (ri == RI_THETA_STAGE || ri == RI_THETA_P1 || ri == RI_RHS || ri == RI_SPEC ||
+          (ri >= RI_THETA_S1 && ri < RI_SCAL_S1)) ? FM_THETA
          : ((ri == RI_SCAL_STAGE || ri == RI_SCAL_P1 || (ri >= RI_SCAL_S1 && ri < RI_SCAL_S1 + 4))
                 ? FM_SCAL
-                : (ri == RI_VEL_P1 ? FM_VEL : -1));
+                : (ri == RI_VEL_P1 ? FM_VEL : (ri == RI_PHYS_P1 ? FM_PHYS1 : -1)));
 }
 __host__ __device__ constexpr int ri_rmode(int ri) {
-  return ri == RI_ANY ? -1 : (ri >= RI_THETA_P1 ? RM_P1 : RM_STAGE);
+  return ri == RI_ANY ? -1
+         : ri == RI_RHS ? RM_RHS
+         : ri == RI_SPEC ? RM_SPEC : (ri >= RI_THETA_P1 ? RM_P1 : RM_STAGE);
 }
 __host__ __device__ constexpr int ri_stage(int ri) {
   return (ri >= RI_THETA_S1 && ri < RI_SCAL_S1) ? ri - RI_THETA_S1 + 1
-         : ((ri >= RI_SCAL_S1 && ri < RI_SCAL_S1 + 4) ? ri - RI_SCAL_S1 + 1 : 0);
+         : ((ri >= RI_SCAL_S1 && ri < RI_SCAL_S1 + 4) ? ri - RI_SCAL_S1 + 1 : (ri == RI_RHS ? 1 : 0));
 }
 enum AlphaKind { AK_GENERAL = 0, AK_ZERO = 1, AK_ONE = 2, AK_HALF = 3, AK_THREEHALF = 4, AK_TWO = 5, AK_MINUSONE = 6 };
 enum StageWrite { SW_NONE = 0, SW_FULL = 1, SW_RING = 2 };
@@ -76,6 +95,7 @@ struct KP {
   double kval;        // 1 / (N dx): fftfreq's scale (the hot kernels compute k from it)
   const void* tw;     // twiddles exp(-2 pi i k/N), plan precision
   const RowTab* rows;
+  int pmax, s2;       // the band (above); N/2 and a bound never met: no pruning of the Jacobian rows
   double inv_n2;      // 1/N^2
   double alpha;
   int akind;
@@ -111,6 +131,9 @@ struct RowArgs {
   void* src_out[4];
   double gx[4], gy[4];
   int rpc;                        // row pairs per CTA (0: the compiled maximum RPC)
+  int st_zero;                    // 1: st_out is read outside the passes (zeros stored outside the band too)
+  unsigned char* tl;              // out-of-band flags of the field's row pairs (null: every row takes every mode)
+  const unsigned char* tl_src;    // flags of src_h's rows (the theta its velocity came from)
 };
 
 // ---- asynchronous global -> shared copies (cp.async) ----
@@ -160,60 +183,141 @@ constexpr int row_min_blocks(int threads) {
 
 __device__ __forceinline__ int mode_abs(int i, int N) { return i <= (N >> 1) ? i : N - i; }
 
-// |k|^-alpha with k = 0 -> 0 (operators.py:134-155)
 // Wavenumber of index i computed in registers with numpy's operation order
 // for fftfreq(N, L/N) * 2 pi, ((m * val) * 2) * pi, so it equals the k1d table
 // bit for bit without a global load per element.
-__device__ __forceinline__ double wavenumber(const KP& kp, int i) {
-  const int m = i <= ((kp.N - 1) >> 1) ? i : i - kp.N;
+__device__ __forceinline__ double wavenumber_m(const KP& kp, int m) {  // m: signed mode number
   return __dmul_rn(__dmul_rn(__dmul_rn((double)m, kp.kval), 2.0), 3.141592653589793116);
+}
+__device__ __forceinline__ double wavenumber(const KP& kp, int i) {
+  return wavenumber_m(kp, i <= ((kp.N - 1) >> 1) ? i : i - kp.N);
 }
 
 // The wavenumber in the arithmetic's precision for the spectral
 // multipliers: float64 (then rounded) in double; in float, the same product
 // in float arithmetic (within an ulp of the rounded float64 value).
 template <typename T>
-__device__ __forceinline__ T wavenumber_t(const KP& kp, int i) {
-  if constexpr (sizeof(T) == 8) {
-    return wavenumber(kp, i);
-  } else {
-    const int m = i <= ((kp.N - 1) >> 1) ? i : i - kp.N;
-    return (float)m * (float)(kp.kval * 6.283185307179586232);
-  }
+__device__ __forceinline__ T wavenumber_mt(const KP& kp, int m) {
+  if constexpr (sizeof(T) == 8) return wavenumber_m(kp, m);
+  else return (float)m * (float)(kp.kval * 6.283185307179586232);
 }
 
-template <typename T>
-__device__ __forceinline__ T inv_frac(T k2, T alpha, int kind) {
-  if (!(k2 > (T)0)) return (T)0;
+// Element m of a row pass's thread: iy = j + m G.  Its mode number, the mode
+// number's magnitude and the mirrored element N - iy, written so that m (a
+// constant of the unrolled loops) decides what is known of them.
+template <int N, int R> struct RowElem {
+  static constexpr int G = N / R;
+  static __device__ __forceinline__ int mode(int j, int m) { return m < R / 2 ? j + m * G : j + m * G - N; }
+  static __device__ __forceinline__ int mag(int j, int m) { return m < R / 2 ? j + m * G : N - m * G - j; }
+  static __device__ __forceinline__ int mirror(int j, int m) { return m == 0 ? (N - j) & (N - 1) : N - m * G - j; }
+};
+// The thread's elements of rows p and pp = N - p of an N x N (or half) array:
+// at(b, m) = (p, iy), mir(b, m) = (pp, N - iy).  OFF: an array's base plus one
+// 32-bit byte offset of the thread plus a constant of m, which keeps the
+// addresses of the multi-size and batch passes, whose arrays' bases come from
+// memory, down to one addition (theta row pass of 96 members 106 -> 87 us); the
+// passes of one field do better with plain indexing (N = 4096 FP32 input pass
+// 122 -> 113 us).
+template <typename C, int N, int R, bool OFF> struct RowPtr {
+  using E = RowElem<N, R>;
+  int p, pp, j;
+  uint32_t o1, o2, o2z;
+  __device__ __forceinline__ RowPtr(int p_, int pp_, int j_)
+      : p(p_), pp(pp_), j(j_),
+        o1((uint32_t)(p_ * N + j_) * sizeof(C)),
+        o2((uint32_t)(pp_ * N + N - j_) * sizeof(C)),
+        o2z((uint32_t)(pp_ * N + ((N - j_) & (N - 1))) * sizeof(C)) {}
+  template <typename B> using Elem = std::conditional_t<std::is_const<B>::value, const C, C>;
+  template <typename B> using Byte = std::conditional_t<std::is_const<B>::value, const char, char>;
+  template <typename B> __device__ __forceinline__ auto at(B* b, int m) const {
+    if constexpr (OFF)
+      return reinterpret_cast<Elem<B>*>(reinterpret_cast<Byte<B>*>(b) + (size_t)o1 + (ptrdiff_t)m * (E::G * (int)sizeof(C)));
+    else
+      return reinterpret_cast<Elem<B>*>(b) + (size_t)p * N + j + m * E::G;
+  }
+  template <typename B> __device__ __forceinline__ auto mir(B* b, int m) const {
+    if constexpr (OFF)
+      return reinterpret_cast<Elem<B>*>(reinterpret_cast<Byte<B>*>(b) + (size_t)(m == 0 ? o2z : o2) -
+                                        (ptrdiff_t)m * (E::G * (int)sizeof(C)));
+    else
+      return reinterpret_cast<Elem<B>*>(b) + (size_t)pp * N + E::mirror(j, m);
+  }
+};
+
+// The general power, and in double the less usual kinds, are calls (pow
+// inlined at every element took more code than the rest of the pass).
+__device__ __noinline__ inline float gen_pow(float x, float y) { return powf(x, y); }
+__device__ __noinline__ inline double gen_frac(double k2, double alpha, int kind) {
+  if (kind == AK_ZERO) return 1.0;
+  if (kind == AK_TWO) return 1.0 / k2;
+  const double k = sqrt(k2);
+  if (kind == AK_THREEHALF) return 1.0 / (k * sqrt(k));
+  if (kind == AK_MINUSONE) return k;
+  return pow(k, -alpha);
+}
+
+// |k|^-alpha of a thread's R modes from their k^2 (0 at k = 0), with one
+// branch on the kind of alpha for all of them: the row passes of up to
+// N = 1024 run as one wave of blocks, each instruction fetched once, so code
+// that is skipped costs nearly as much as code that runs.
+template <typename T, int R>
+__device__ __forceinline__ void inv_frac(const T (&k2)[R], T alpha, int kind, T (&out)[R]) {
+  auto each = [&](auto f) {
+#pragma unroll
+    for (int m = 0; m < R; ++m) out[m] = f(k2[m]);
+  };
   if constexpr (sizeof(T) == 4) {
     // single precision: the hardware reciprocal square root (about 2 ulp)
     // instead of correctly rounded square roots and divisions
-    const float r1 = rsqrtf(k2);  // 1 / |k|
-    switch (kind) {
-      case AK_ZERO: return 1.f;
-      case AK_ONE: return r1;
-      case AK_HALF: return rsqrtf(k2 * r1);             // |k|^-1/2
-      case AK_THREEHALF: return r1 * rsqrtf(k2 * r1);   // |k|^-3/2
-      case AK_TWO: return r1 * r1;
-      case AK_MINUSONE: return k2 * r1;
-      default: return powf(k2 * r1, -alpha);
-    }
+    if (kind == AK_ONE) each([](float x) { return rsqrtf(x); });
+    else if (kind == AK_HALF) each([](float x) { return rsqrtf(x * rsqrtf(x)); });
+    else if (kind == AK_ZERO) each([](float) { return 1.f; });
+    else if (kind == AK_THREEHALF) each([](float x) { const float r = rsqrtf(x); return r * rsqrtf(x * r); });
+    else if (kind == AK_TWO) each([](float x) { const float r = rsqrtf(x); return r * r; });
+    else if (kind == AK_MINUSONE) each([](float x) { return x * rsqrtf(x); });
+    else each([&](float x) { return gen_pow(x * rsqrtf(x), -alpha); });
+  } else {
+    if (kind == AK_ONE) each([](double x) { return 1.0 / sqrt(x); });
+    else if (kind == AK_HALF) each([](double x) { return 1.0 / sqrt(sqrt(x)); });
+    else each([&](double x) { return gen_frac(x, alpha, kind); });
   }
-  switch (kind) {
-    case AK_ZERO: return (T)1;
-    case AK_ONE: return (T)1 / sqrt(k2);
-    case AK_HALF: return (T)1 / sqrt(sqrt(k2));
-    case AK_THREEHALF: { T k = sqrt(k2); return (T)1 / (k * sqrt(k)); }
-    case AK_TWO: return (T)1 / k2;
-    case AK_MINUSONE: return sqrt(k2);
-    default: return pow(sqrt(k2), -alpha);
-  }
+#pragma unroll
+  for (int m = 0; m < R; ++m)
+    if (!(k2[m] > (T)0)) out[m] = (T)0;
 }
 
 __device__ __forceinline__ double kpow(double k2, int p) {
   // k2^(p/2) for p in {2, 4, 8}
   double k4 = k2 * k2;
   return p == 2 ? k2 : (p == 4 ? k4 : k4 * k4);
+}
+
+// Diagonal linear operator of a mode in float64: L, or exp(L dt/2) where
+// use_exp is set.  kind: 0 theta, 3 theta with the drag, 2 a scalar, 1 the
+// solver's hyperviscosity alone (solver.py:28-58).
+__device__ __forceinline__ double linear_op(const KP& kp, double kxd, int m, int kind, double kappa, bool use_exp) {
+  const double kyd = wavenumber_m(kp, m);
+  const double k2d = kxd * kxd + kyd * kyd;
+  double Ld;
+  if (kind == 2) {
+    Ld = -kappa * k2d;
+  } else {
+    Ld = -kp.nu_s * kpow(k2d, kp.ps);
+    if (kind != 1) {
+      Ld = Ld - kp.nu_d * kpow(k2d, kp.pd);
+      if (kind == 3) Ld -= kp.mu;
+    }
+  }
+  if (!use_exp) return Ld;
+  const double x = Ld * (0.5 * kp.dt);
+  return x < -745.0 ? 0.0 : exp(x);
+}
+
+// The same as a call, for passes that are bound by fetching their code once
+// (it would otherwise stand at every element, float64 exponential included).
+__device__ __noinline__ inline double linear_op_call(const KP& kp, double kxd, int m, int kind, double kappa,
+                                                     bool use_exp) {
+  return linear_op(kp, kxd, m, kind, kappa, use_exp);
 }
 
 template <typename C>
@@ -227,6 +331,20 @@ __device__ __forceinline__ int ring_ord(const RowTab& rt, int iy) {
     return rt.row_start + npos + (iy - rt.neg_lo);
   }
   return -1;
+}
+
+// Scaled ring forcing of stage s at (row of rt, iy), zero off the ring; and as
+// a call (see linear_op_call).
+template <typename C>
+__device__ __forceinline__ C ring_force(const KP& kp, const RowTab& rt, int iy, int s) {
+  const int o = ring_ord(rt, iy);
+  if (o < 0) return mkc<C>(0, 0);
+  const double2 f = kp.ringF[(size_t)(s - 1) * kp.n_ring + o];
+  return mkc<C>(f.x, f.y);
+}
+template <typename C>
+__device__ __noinline__ C ring_force_call(const KP& kp, const RowTab* rt, int iy, int s) {
+  return ring_force<C>(kp, *rt, iy, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,8 +369,8 @@ __host__ __device__ constexpr int fs_kind(int fs, int f) {
 
 // The fields of set FS of the row pair's mode: form their spectra from
 // theta_{s+1} at (p, iy) / (N-p, N-iy), transform them together along y and
-// write xh[f0 + f][p][:].
-template <typename T, int LOG2N, int R, int FS, typename HA>
+// write xh[f0 + f][p][:].  SRC: also the mean-gradient sources (velocity pass).
+template <typename T, int LOG2N, int R, int FS, bool SRC, bool OFF, typename HA>
 __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha, int f0, int j, int p, bool valid,
                                            typename Cplx<T>::type* wbuf) {
   using C = typename Cplx<T>::type;
@@ -260,21 +378,32 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
   constexpr int NF = fs_fields(FS);
   constexpr bool uv = FS == FS_UV || FS == FS_ALL;  // u and v: the multiplier |k|^-alpha
   const C* __restrict__ tw = reinterpret_cast<const C*>(kp.tw);
-  const T kx = wavenumber_t<T>(kp, p);
+  using E = RowElem<N, R>;
+  const T kx = wavenumber_mt<T>(kp, p < H ? p : p - N);
   const T s_n2 = (T)kp.inv_n2;
   const T dkx = (p == H) ? (T)0 : kx;
   const T nkx = (p == H) ? kx : (T)0;
   C V[NF][R];
+  T frac[R];
+  if constexpr (uv) {
+    T k2[R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      const T ky = wavenumber_mt<T>(kp, E::mode(j, m));
+      k2[m] = kx * kx + ky * ky;
+    }
+    inv_frac<T, R>(k2, (T)kp.alpha, kp.akind, frac);
+  }
 #pragma unroll
   for (int m = 0; m < R; ++m) {
     const int iy = j + m * G;
     C h, an;
     ha(m, h, an);
-    const T ky = wavenumber_t<T>(kp, iy);
+    const T ky = wavenumber_mt<T>(kp, E::mode(j, m));
     const T dky = (iy == H) ? (T)0 : ky;
     const T nky = (iy == H) ? ky : (T)0;
     T mm = (T)0;
-    if constexpr (uv) mm = inv_frac<T>(kx * kx + ky * ky, (T)kp.alpha, kp.akind) * s_n2;
+    if constexpr (uv) mm = frac[m] * s_n2;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       const int kind = fs_kind(FS, f);
@@ -294,7 +423,7 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
       }
       V[f][m] = X;
     }
-    if constexpr (uv) {
+    if constexpr (uv && SRC) {
       if (a.n_src > 0 && valid) {
         // S^ = -N^2 (gx X_u + gy X_v): the mean-gradient scalar sources, from
         // the u and v spectra of this batch
@@ -310,12 +439,14 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
   }
   fft_multi<T, LOG2N, R, +1, NF>(V, wbuf, XB, j, tw);
   if (valid) {
-    C* xh = reinterpret_cast<C*>(a.xh);
-    const size_t fstride = (size_t)(H + 1) * N;
+    constexpr size_t fstride = (size_t)(H + 1) * N;
+    const RowPtr<C, N, R, OFF> at(p, 0, j);
 #pragma unroll
-    for (int f = 0; f < NF; ++f)
+    for (int f = 0; f < NF; ++f) {
+      C* xh = reinterpret_cast<C*>(a.xh) + (f0 + f) * fstride;
 #pragma unroll
-      for (int m = 0; m < R; ++m) xh[(f0 + f) * fstride + (size_t)p * N + j + m * G] = V[f][m];
+      for (int m = 0; m < R; ++m) *at.at(xh, m) = V[f][m];
+    }
   }
 }
 
@@ -323,7 +454,8 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
 // the elements iy = j + m G) have their theta_n / acc values prefetched with
 // cp.async ahead of use; the first DEPTH chunks are requested before the
 // forward FFT of the J row, so their latency hides behind it.
-template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI = RI_ANY>
+// BATCH: a pass of many fields, its arguments read from device arrays.
+template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI = RI_ANY, bool BATCH = RI == RI_ANY>
 __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int tile) {
   // modes fixed by the instance (RI), else read from the arguments
   const int rmode = ri_rmode(RI) >= 0 ? ri_rmode(RI) : a.rmode;
@@ -352,214 +484,304 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   const bool pair = (p != 0) && (p != H);
   const C* __restrict__ tw = reinterpret_cast<const C*>(kp.tw);
   const RowTab rt = kp.rows[p];
+  const int band2 = p <= kp.pmax ? kp.s2 - p * p : -1;  // in the band: m_y^2 <= band2
+  using EL = RowElem<N, R>;
+  const RowPtr<C, N, R, BATCH> rp(p, pp, j);
+  auto in_band = [&](int m) { const int my = EL::mag(j, m); return my * my <= band2; };
+  const bool tile_out = tile * rpc > kp.pmax;  // every row of the block lies beyond the band
   const double kxd = wavenumber(kp, p);
   const T kx = (T)kxd;
   const T s_n2 = (T)kp.inv_n2;
-  bool bad = false;
+  bool bad = false, skip_p1 = false;
+  __shared__ bool warp_out[32];  // RM_P1: a warp saw a mode outside the band
 
   C v[R];   // FFT registers
   C t1[R];  // theta_{s+1} (or theta_in) at e1 = (p, iy)
   C t2[R];  // theta_{s+1} at e2 = (pp, N - iy)
 
   if (rmode == RM_P1) {
-    const C* th = reinterpret_cast<const C*>(a.th_n);
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      const int iy = j + m * G;
-      const int iyp = (N - iy) & (N - 1);
-      t1[m] = th[(size_t)p * N + iy];
-      t2[m] = th[(size_t)pp * N + iyp];
+      t1[m] = *rp.at(a.th_n, m);
+      t2[m] = *rp.mir(a.th_n, m);
+    }
+    if (a.tl) {
+      bool out = false;
+#pragma unroll
+      for (int m = 0; m < R; ++m)
+        out |= !in_band(m) && !(t1[m].x == (T)0 && t1[m].y == (T)0 && t2[m].x == (T)0 && t2[m].y == (T)0);
+      // flags are of the block's rows together: at once when the block may
+      // leave, else collected by warp and stored after the transforms
+      if (tile_out) {
+        const int any = __syncthreads_or(out);
+        if (valid && j == 0) a.tl[p] = any ? 1 : 0;
+        if (!any) return;
+      } else {
+        const bool w = __any_sync(__activemask(), out);
+        if ((threadIdx.x & 31) == 0) warp_out[threadIdx.x >> 5] = w;
+      }
     }
   } else {
-    // stage pass: request this thread's theta_n / acc elements of the first
-    // DEPTH chunks (own slots only, so no barrier is needed to consume them)
-    const bool pf_th = rmode == RM_STAGE && stage <= 3;
-    const bool pf_acc = rmode == RM_STAGE && stage >= 2;
-    const C* pth = reinterpret_cast<const C*>(a.th_n);
-    const C* pacc = reinterpret_cast<const C*>(a.acc);
-    auto issue = [&](int m) {
-      const int iy = j + m * G;
-      const int iyp = (N - iy) & (N - 1);
-      C* slot = pf + (size_t)(m % DEPTH) * 4 * G + j;
-      if (pf_th) {
-        cp_async_elem(slot, pth + (size_t)p * N + iy, (int)sizeof(C));
-        if (pair) cp_async_elem(slot + G, pth + (size_t)pp * N + iyp, (int)sizeof(C));
+    // Whether this row (and any row of the block, block-uniform) has modes
+    // outside the band, or its source does.
+    bool tail = a.tl == nullptr || a.extra != nullptr, src_row = true;
+    bool tile_tail = tail;
+    if (a.tl && rmode != RM_SPEC) {
+      for (int g = 0; g < rpc; ++g) {
+        const int pg = tile * rpc + g <= H ? tile * rpc + g : H;
+        bool t = a.tl[pg] != 0;
+        if (a.tl_src) {
+          const bool ts = a.tl_src[pg] != 0;
+          if (pg == p) src_row = ts || p <= kp.pmax;  // unwritten source rows are zero
+          t |= ts;
+        }
+        if (pg == p) tail |= t;
+        tile_tail |= t;
       }
-      if (pf_acc) {
-        cp_async_elem(slot + 2 * G, pacc + (size_t)p * N + iy, (int)sizeof(C));
-        if (pair) cp_async_elem(slot + 3 * G, pacc + (size_t)pp * N + iyp, (int)sizeof(C));
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int m = 0; m < DEPTH; ++m) issue(m);
-    // forward DFT along y of the x-transformed Jacobian row p
-    const C* jh = reinterpret_cast<const C*>(a.jh);
-#pragma unroll
-    for (int m = 0; m < R; ++m) v[m] = jh[(size_t)p * N + j + m * G];
-    fft_group<T, LOG2N, R, -1>(v, wbuf, j, tw);
-    // v[m] = J^(p, iy) ; J^(pp, N - iy) = conj(v[m])
-    if (rmode == RM_SPEC) {
-      // forward transform of a real field: rows p and N - p of its spectrum
-      C* out = reinterpret_cast<C*>(a.rhs_out);
-      if (valid) {
+    }
+    if (tile_out && !tile_tail && rmode != RM_SPEC) {
+      // every mode of the block's rows is zero and stays zero
+      void* z1 = rmode == RM_RHS ? a.rhs_out
+                 : stage == 4    ? (a.th_out != a.th_n ? a.th_out : nullptr)
+                                 : (a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
+      if (z1 && valid) {
 #pragma unroll
         for (int m = 0; m < R; ++m) {
-          const int iy = j + m * G;
-          out[(size_t)p * N + iy] = v[m];
-          if (pair) out[(size_t)pp * N + ((N - iy) & (N - 1))] = cconj(v[m]);
+          *rp.at(z1, m) = mkc<C>(0, 0);
+          if (pair) *rp.mir(z1, m) = mkc<C>(0, 0);
         }
       }
       return;
     }
+    // request this thread's theta_n / acc elements of the first DEPTH chunks
+    // (own slots only, so no barrier is needed to consume them): those in the
+    // band at once, the others once the row's flag has arrived
+    const bool pf_th = rmode == RM_STAGE && stage <= 3;
+    const bool pf_acc = rmode == RM_STAGE && stage >= 2;
+    auto issue = [&](int m) {
+      C* slot = pf + (size_t)(m % DEPTH) * 4 * G + j;
+      if (pf_th) {
+        cp_async_elem(slot, rp.at(a.th_n, m), (int)sizeof(C));
+        if (pair) cp_async_elem(slot + G, rp.mir(a.th_n, m), (int)sizeof(C));
+      }
+      if (pf_acc) {
+        cp_async_elem(slot + 2 * G, rp.at(a.acc, m), (int)sizeof(C));
+        if (pair) cp_async_elem(slot + 3 * G, rp.mir(a.acc, m), (int)sizeof(C));
+      }
+    };
+#pragma unroll
+    for (int m = 0; m < DEPTH; ++m)
+      if (in_band(m)) issue(m);
+    // forward DFT along y of the x-transformed Jacobian row p (the column pass
+    // leaves the rows beyond the band unwritten: the mask discards them)
+    const bool use_j = rmode == RM_SPEC || !tile_out;
+#pragma unroll
+    for (int m = 0; m < R; ++m) v[m] = use_j ? *rp.at(a.jh, m) : mkc<C>(0, 0);
+#pragma unroll
+    for (int m = 0; m < DEPTH; ++m)
+      if (tail && !in_band(m)) issue(m);
+    cp_async_commit();  // the first DEPTH chunks are one group, each later chunk one
     const int s = stage;
     const bool scal = fmode == FM_SCAL;
-    const C* st_in = reinterpret_cast<const C*>(s == 1 ? a.th_n : a.st_in);
-    C* acc = reinterpret_cast<C*>(a.acc);
-    C* st_out = reinterpret_cast<C*>(a.st_out);
-    C* th_out = reinterpret_cast<C*>(a.th_out);
-    const C* extra = reinterpret_cast<const C*>(a.extra);
-    const C* src_h = reinterpret_cast<const C*>(a.src_h);
     const double dt = kp.dt;
     const bool explicit_lin = (kp.scheme == 0);
+    // lt = L for the explicit scheme (and the right-hand side); e = exp(L dt/2)
+    // and e2 = e^2 for the integrating-factor form, whose last stage, th_{n+1} =
+    // acc + dt/6 k, does not use them
+    const bool use_exp = rmode == RM_STAGE && !explicit_lin && s < 4;
+    const bool use_lin = rmode == RM_RHS || explicit_lin || s < 4;
+    constexpr bool CALLS = LOG2N <= 9 || BATCH;
+    auto linear = [&](int m, T& e, T& e2, T& lt) {
+      e = e2 = (T)1;
+      lt = (T)0;
+      if (!use_lin) return;
+      const int kind = rmode == RM_RHS ? 1 : scal ? 2 : EL::mag(j, m) <= rt.dragmax ? 3 : 0;
+      const double x = CALLS ? linear_op_call(kp, kxd, EL::mode(j, m), kind, a.kappa, use_exp)
+                             : linear_op(kp, kxd, EL::mode(j, m), kind, a.kappa, use_exp);
+      if (use_exp) {
+        e = (T)x;
+        e2 = (T)(x * x);
+      } else {
+        lt = (T)x;
+      }
+    };
+    // The radix-4 passes are bound by the latency of their one wave of blocks:
+    // they evaluate the operator for all their elements ahead of the transform
+    // (independent chains, while the loads are under way) and update them
+    // without branches.  The radix-8 passes, short of registers and with more
+    // warps to hide a chain, branch around each element outside the band.
+    constexpr bool HOIST = R == 4 && sizeof(T) == 4 && !BATCH;
+    constexpr bool FLAT = HOIST || sizeof(T) == 8;
+    T fe[HOIST ? R : 1], fe2[HOIST ? R : 1], fl[HOIST ? R : 1];
+    if constexpr (HOIST) {
+#pragma unroll
+      for (int m = 0; m < R; ++m) linear(m, fe[m], fe2[m], fl[m]);
+    }
+    if (use_j) fft_group<T, LOG2N, R, -1>(v, wbuf, j, tw);
+    // v[m] = J^(p, iy) ; J^(pp, N - iy) = conj(v[m])
+    if (rmode == RM_SPEC) {
+      // forward transform of a real field: rows p and N - p of its spectrum
+      if (valid) {
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          *rp.at(a.rhs_out, m) = v[m];
+          if (pair) *rp.mir(a.rhs_out, m) = cconj(v[m]);
+        }
+      }
+      return;
+    }
+    const void* st_in = s == 1 ? a.th_n : a.st_in;
     // the scalar's source term is read one chunk ahead, ahead of the wait
     // for the chunk's prefetched values, so that its latency overlaps the
     // element updates of the chunk before
-    const bool use_src = scal && src_h != nullptr;
+    const bool use_src = scal && a.src_h != nullptr && src_row;
     C sh_next = mkc<C>(0, 0);
-    if (use_src) sh_next = src_h[(size_t)p * N + j];
+    if (use_src) sh_next = *rp.at(a.src_h, 0);
+    // the explicit scheme's stage input likewise
+    const bool use_st = (explicit_lin && s > 1 && rmode == RM_STAGE) || rmode == RM_RHS;
+    C x_next1 = mkc<C>(0, 0), x_next2 = mkc<C>(0, 0);
+    auto load_st = [&](int m) {
+      if (use_st && (tail || in_band(m))) {
+        x_next1 = *rp.at(st_in, m);
+        if (pair) x_next2 = *rp.mir(st_in, m);
+      }
+    };
+    load_st(0);
+    bool out_nz = false;  // a non-zero new mode outside the band
+    // where the zeros outside the band have to be stored
+    void* zero_out = rmode == RM_RHS ? a.rhs_out
+                     : s == 4 ? (a.th_out != a.th_n ? a.th_out : nullptr)
+                              : (a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
+    const bool ring_row = !scal && kp.ring_on && (rt.pos_lo <= rt.pos_hi || rt.neg_lo <= rt.neg_hi);
+    const T tdt = (T)dt, dt2 = tdt * (T)0.5, dt3 = tdt / (T)3, dt6 = tdt / (T)6;
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      const int iy = j + m * G;
-      const int iyp = (N - iy) & (N - 1);
-      const size_t e1 = (size_t)p * N + iy;
-      const size_t e2 = (size_t)pp * N + iyp;
-      const int my = mode_abs(iy, N);
+      const int my = EL::mag(j, m);
       const C sh = sh_next;
-      if (use_src && m + 1 < R) sh_next = src_h[(size_t)p * N + iy + G];
-      cp_async_wait<DEPTH - 1>();  // chunk m has landed (groups are issued in order)
-      const C* slot = pf + (size_t)(m % DEPTH) * 4 * G + j;
-      const double kyd = wavenumber(kp, iy);
-      const double k2d = kxd * kxd + kyd * kyd;
-      // diagonal linear operator in float64 (the integrating-factor form's
-      // last stage, th_{n+1} = acc + dt/6 k, does not use it)
-      double Ld = 0.0;
-      if (explicit_lin || s < 4) {
-        if (scal) {
-          Ld = -a.kappa * k2d;
+      if (use_src && m + 1 < R) sh_next = *rp.at(a.src_h, m + 1);
+      const C xi1 = x_next1, xi2 = x_next2;
+      if (m + 1 < R) load_st(m + 1);
+      // chunk m has landed (groups complete in order)
+      if (m == 0) cp_async_wait<0>();
+      else if (m >= DEPTH) cp_async_wait<DEPTH - 1>();
+      const bool inb = in_band(m);
+      const bool act = inb || tail;  // else zero, and stays zero
+      C o1 = mkc<C>(0, 0), o2 = mkc<C>(0, 0);  // theta_{s+1} (or theta_{n+1})
+      if (FLAT || act) {
+        const C* slot = pf + (size_t)(m % DEPTH) * 4 * G + j;
+        const bool wr = valid && act;
+        T E, E2, Lt;
+        if constexpr (HOIST) {
+          E = fe[m];
+          E2 = fe2[m];
+          Lt = fl[m];
         } else {
-          Ld = -kp.nu_s * kpow(k2d, kp.ps) - kp.nu_d * kpow(k2d, kp.pd);
-          if (my <= rt.dragmax) Ld -= kp.mu;
+          linear(m, E, E2, Lt);
         }
-      }
-      const T dmask = (my <= rt.dmax) ? (T)1 : (T)0;
-      C J1 = v[m];
-      C n1 = mkc<C>(-dmask * J1.x, -dmask * J1.y);
-      C n2 = mkc<C>(-dmask * J1.x, dmask * J1.y);  // conj
-      if (use_src) {
-        n1 = cadd(n1, sh);
-        n2 = cadd(n2, cconj(sh));
-      }
-      int ord1 = -1, ord2 = -1;
-      if (!scal && kp.ring_on) {
-        ord1 = ring_ord(rt, iy);
-        if (ord1 >= 0) {
-          const double2 F1 = kp.ringF[(size_t)(s - 1) * kp.n_ring + ord1];
-          n1.x += (T)F1.x; n1.y += (T)F1.y;
-          if (pair) {
-            ord2 = ring_ord(kp.rows[pp], iyp);
-            if (ord2 >= 0) {
-              const double2 F2 = kp.ringF[(size_t)(s - 1) * kp.n_ring + ord2];
-              n2.x += (T)F2.x; n2.y += (T)F2.y;
-            }
+        // (selected, not multiplied by the mask: rows beyond pmax hold no J)
+        const C J1 = (my <= rt.dmax) ? v[m] : mkc<C>(0, 0);
+        C n1 = mkc<C>(-J1.x, -J1.y);
+        C n2 = mkc<C>(-J1.x, J1.y);  // conj
+        if (use_src) {
+          n1 = cadd(n1, sh);
+          n2 = cadd(n2, cconj(sh));
+        }
+        const int iy = j + m * G;
+        const bool ring = ring_row && ((iy >= rt.pos_lo && iy <= rt.pos_hi) || (iy >= rt.neg_lo && iy <= rt.neg_hi));
+        if (ring) {
+          if constexpr (CALLS) {
+            n1 = cadd(n1, ring_force_call<C>(kp, kp.rows + p, iy, s));
+            if (pair) n2 = cadd(n2, ring_force_call<C>(kp, kp.rows + pp, EL::mirror(j, m), s));
+          } else {
+            n1 = cadd(n1, ring_force<C>(kp, rt, iy, s));
+            if (pair) n2 = cadd(n2, ring_force<C>(kp, kp.rows[pp], EL::mirror(j, m), s));
           }
         }
-      }
-      if (extra) {
-        n1 = cadd(n1, extra[e1]);
-        if (pair) n2 = cadd(n2, extra[e2]);
-      }
-      if (rmode == RM_RHS) {
-        // core RHS (solver.py:28-58): advection + solver hyperviscosity only
-        const C x1 = st_in[e1];
-        const T Ls = (T)(-kp.nu_s * kpow(k2d, kp.ps));
-        C* out = reinterpret_cast<C*>(a.rhs_out);
-        if (valid) out[e1] = cadd(n1, cscale(x1, Ls));
-        if (pair) {
-          const C x2 = st_in[e2];
-          if (valid) out[e2] = cadd(n2, cscale(x2, Ls));
+        if (a.extra) {
+          n1 = cadd(n1, *rp.at(a.extra, m));
+          if (pair) n2 = cadd(n2, *rp.mir(a.extra, m));
         }
-        if (m + DEPTH < R) issue(m + DEPTH);
-        else cp_async_commit();
-        continue;
-      }
-      C k1v = n1, k2v = n2;
-      C xs1 = mkc<C>(0, 0), xs2 = mkc<C>(0, 0);  // stage input
-      if (s == 1) {
-        xs1 = slot[0];
-        if (pair) xs2 = slot[G];
-      } else if (explicit_lin) {
-        xs1 = st_in[e1];
-        if (pair) xs2 = st_in[e2];
-      }
-      T E = (T)1, E2 = (T)1;
-      if (explicit_lin) {
-        const T Lt = (T)Ld;
-        k1v = cadd(k1v, cscale(xs1, Lt));
-        k2v = cadd(k2v, cscale(xs2, Lt));
-      } else if (s < 4) {
-        const double x = Ld * (0.5 * dt);
-        const double Ed = x < -745.0 ? 0.0 : exp(x);
-        E = (T)Ed;
-        E2 = (T)(Ed * Ed);
-      }
-      const T tdt = (T)dt;
-      C o1, o2 = mkc<C>(0, 0);  // theta_{s+1} (or theta_{n+1})
-      if (s == 1) {
-        // acc = E^2 (th + dt/6 k) ; th2 = E (th + dt/2 k)
-        const C a1 = cscale(cadd(xs1, cscale(k1v, tdt / (T)6)), E2);
-        if (valid) acc[e1] = a1;
-        o1 = cscale(cadd(xs1, cscale(k1v, tdt * (T)0.5)), E);
-        if (pair) {
-          const C a2 = cscale(cadd(xs2, cscale(k2v, tdt / (T)6)), E2);
-          if (valid) acc[e2] = a2;
-          o2 = cscale(cadd(xs2, cscale(k2v, tdt * (T)0.5)), E);
-        }
-      } else if (s == 2 || s == 3) {
-        C a1 = slot[2 * G];
-        a1 = cadd(a1, cscale(k1v, tdt / (T)3 * E));
-        if (valid) acc[e1] = a1;
-        const C x1 = slot[0];
-        if (s == 2) o1 = cadd(cscale(x1, E), cscale(k1v, tdt * (T)0.5));   // th3 = E th + dt/2 k
-        else        o1 = cadd(cscale(x1, E2), cscale(k1v, tdt * E));       // th4 = E^2 th + dt E k
-        if (pair) {
-          C a2 = slot[3 * G];
-          a2 = cadd(a2, cscale(k2v, tdt / (T)3 * E));
-          if (valid) acc[e2] = a2;
-          const C x2 = slot[G];
-          if (s == 2) o2 = cadd(cscale(x2, E), cscale(k2v, tdt * (T)0.5));
-          else        o2 = cadd(cscale(x2, E2), cscale(k2v, tdt * E));
-        }
-      } else {
-        // th_{n+1} = acc + dt/6 k
-        o1 = cadd(slot[2 * G], cscale(k1v, tdt / (T)6));
-        if (valid) th_out[e1] = o1;
-        if (pair) {
-          o2 = cadd(slot[3 * G], cscale(k2v, tdt / (T)6));
-          if (valid) th_out[e2] = o2;
+        if (rmode == RM_RHS) {
+          if (wr) {
+            *rp.at(a.rhs_out, m) = cadd(n1, cscale(xi1, Lt));
+            if (pair) *rp.mir(a.rhs_out, m) = cadd(n2, cscale(xi2, Lt));
+          }
+        } else {
+          C k1v = n1, k2v = n2;
+          C xs1 = xi1, xs2 = xi2;  // stage input
+          if (s == 1) {
+            xs1 = slot[0];
+            if (pair) xs2 = slot[G];
+          }
+          if (explicit_lin) {
+            k1v = cadd(k1v, cscale(xs1, Lt));
+            k2v = cadd(k2v, cscale(xs2, Lt));
+          }
+          if (s == 1) {
+            // acc = E^2 (th + dt/6 k) ; th2 = E (th + dt/2 k)
+            const C a1 = cscale(cadd(xs1, cscale(k1v, dt6)), E2);
+            if (wr) *rp.at(a.acc, m) = a1;
+            o1 = cscale(cadd(xs1, cscale(k1v, dt2)), E);
+            if (pair) {
+              const C a2 = cscale(cadd(xs2, cscale(k2v, dt6)), E2);
+              if (wr) *rp.mir(a.acc, m) = a2;
+              o2 = cscale(cadd(xs2, cscale(k2v, dt2)), E);
+            }
+          } else if (s == 2 || s == 3) {
+            C a1 = slot[2 * G];
+            a1 = cadd(a1, cscale(k1v, dt3 * E));
+            if (wr) *rp.at(a.acc, m) = a1;
+            const C x1 = slot[0];
+            if (s == 2) o1 = cadd(cscale(x1, E), cscale(k1v, dt2));   // th3 = E th + dt/2 k
+            else        o1 = cadd(cscale(x1, E2), cscale(k1v, tdt * E));       // th4 = E^2 th + dt E k
+            if (pair) {
+              C a2 = slot[3 * G];
+              a2 = cadd(a2, cscale(k2v, dt3 * E));
+              if (wr) *rp.mir(a.acc, m) = a2;
+              const C x2 = slot[G];
+              if (s == 2) o2 = cadd(cscale(x2, E), cscale(k2v, dt2));
+              else        o2 = cadd(cscale(x2, E2), cscale(k2v, tdt * E));
+            }
+          } else {
+            // th_{n+1} = acc + dt/6 k
+            o1 = cadd(slot[2 * G], cscale(k1v, dt6));
+            if (pair) o2 = cadd(slot[3 * G], cscale(k2v, dt6));
+            if (wr) {
+              *rp.at(a.th_out, m) = o1;
+              if (pair) *rp.mir(a.th_out, m) = o2;
+            }
+          }
+          if (FLAT && !act) o1 = o2 = mkc<C>(0, 0);
+          if (s < 4 && wr) {
+            if (a.stage_write == SW_FULL || (a.stage_write == SW_RING && ring)) {
+              *rp.at(a.st_out, m) = o1;
+              if (pair) *rp.mir(a.st_out, m) = o2;
+            }
+          }
+          bad |= !(cfinite(o1) && cfinite(o2));
+          if (!inb) out_nz |= !(o1.x == (T)0 && o1.y == (T)0 && o2.x == (T)0 && o2.y == (T)0);
         }
       }
-      if (s < 4 && valid) {
-        if (a.stage_write == SW_FULL || (a.stage_write == SW_RING && ord1 >= 0)) {
-          st_out[e1] = o1;
-          if (pair) st_out[e2] = o2;
-        }
+      if (!act && zero_out && valid) {
+        *rp.at(zero_out, m) = mkc<C>(0, 0);
+        if (pair) *rp.mir(zero_out, m) = mkc<C>(0, 0);
       }
-      bad |= !(cfinite(o1) && cfinite(o2));
       t1[m] = o1;
       t2[m] = o2;
-      if (m + DEPTH < R) issue(m + DEPTH);
-      else cp_async_commit();  // empty group keeps the in-order accounting
+      if (m + DEPTH < R && (tail || in_band(m + DEPTH))) issue(m + DEPTH);
+      if constexpr (DEPTH < R) cp_async_commit();  // (empty groups keep the in-order accounting)
+    }
+    if (a.tl && tile_tail && a.do_p1 && rmode == RM_STAGE) {
+      // flags of theta_{s+1}'s rows: after the last stage those of the next
+      // step; before it a row stays with every mode once it holds any (its
+      // source or extra term put some there)
+      if (s == 4 && !a.extra) {
+        const int any = __syncthreads_or(out_nz);
+        if (valid && j == 0) a.tl[p] = any ? 1 : 0;
+        skip_p1 = !any && tile_out;
+      } else if (tail && valid && j == 0) {
+        a.tl[p] = 1;
+      }
     }
   }
   if (kp.status) {
@@ -568,10 +790,10 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   // NFX = 0 is the instantiation for stage passes without the inverse
   // transforms (the last stage of a step): compiled without them, it needs
   // few registers and one exchange buffer, so two blocks share an SM.
-  if constexpr (NFX == 0) {
+  if constexpr (NFX == 0 || ri_rmode(RI) == RM_RHS || ri_rmode(RI) == RM_SPEC) {
     return;
   } else {
-  if (!a.do_p1) return;
+  if (!a.do_p1 || skip_p1) return;
 
   // Rows 0 and N/2 pair with themselves: e2 = (p, N - iy) is owned by another
   // thread of the group, so its new value is exchanged through shared memory
@@ -627,21 +849,26 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   auto fields = [&](auto ha) {
     if (fmode == FM_THETA) {
       if constexpr (NFT == 4) {
-        row_fields<T, LOG2N, R, FS_ALL>(kp, a, ha, 0, j, p, valid, wbuf);
+        row_fields<T, LOG2N, R, FS_ALL, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
       } else {
-        row_fields<T, LOG2N, R, FS_UV>(kp, a, ha, 0, j, p, valid, wbuf);
-        row_fields<T, LOG2N, R, FS_GRAD>(kp, a, ha, 2, j, p, valid, wbuf);
+        row_fields<T, LOG2N, R, FS_UV, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
+        row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 2, j, p, valid, wbuf);
       }
     } else if (fmode == FM_PHYS1) {
-      row_fields<T, LOG2N, R, FS_ID>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_ID, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
     } else if (fmode == FM_VEL) {
-      row_fields<T, LOG2N, R, FS_UV>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_UV, RI == RI_VEL_P1, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
     } else {
-      row_fields<T, LOG2N, R, FS_GRAD>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
     }
   };
   if constexpr (nfx_park(NFX)) fields(ha_smem);
   else fields(ha_reg);
+  if (rmode == RM_P1 && a.tl && !tile_out && valid && j == 0) {
+    bool any = false;  // (the transforms' barriers lie between)
+    for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) any |= warp_out[w];
+    a.tl[p] = any ? 1 : 0;
+  }
   }
 }
 
@@ -686,6 +913,8 @@ struct ColArgs {
   int ring_ou;
   int herm_ord[4];          // ordinals of (0,0),(N/2,0),(0,N/2),(N/2,N/2) or -1
   double* ring_scale_out;   // [4]
+  const unsigned char* tl;  // out-of-band flags of xh's rows: rows beyond pmax with flag 0 are zero and
+  const unsigned char* tl2; // unwritten (null: every row is written); of xh2's rows
   int np;                   // column pairs per CTA (0: the compiled maximum NP)
   int tma;                  // 1: the half columns of xh arrive as TMA tiles through the
                             // kernel's tensor map (fields 0.. of the map = xh + f (N/2+1) N)
@@ -728,8 +957,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-// Issue the copies of the half columns of field f for every column pair of
-// the block into buffer slot `buf` of each group (no registers, no wait).
+// Issue the copies of rows r0..r1 of the half columns of field f for every
+// column pair of the block into buffer slot `buf` of each group (no registers,
+// no wait).  With tiles, r0 = 0 takes whole boxes up to the one that holds r1,
+// and r0 > 0 the boxes after the one that holds r0 - 1.
 // A row of a column pair is 2 sizeof(C) contiguous bytes (one 16-byte copy in
 // float, two in double).  Copy unit u = (row kx, pair q, part): part fastest,
 // then the pair, so consecutive threads read a row's 16 np contiguous bytes
@@ -742,8 +973,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 // pair and 16 bytes, as before.
 template <typename T, int LOG2N, int R, int NP, int NBUF>
 __device__ __forceinline__ void col_fetch(const typename Cplx<T>::type* __restrict__ f, int y0, int buf,
-                                          typename Cplx<T>::type* smem, int np, const CUtensorMap* tm = nullptr,
-                                          int fidx = 0, uint64_t* bar = nullptr) {
+                                          typename Cplx<T>::type* smem, int np, int r0, int r1,
+                                          const CUtensorMap* tm = nullptr, int fidx = 0, uint64_t* bar = nullptr) {
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N, H = N / 2, SZ = ColBuf<N, R>::SZ;
   constexpr int LC = sizeof(C) == 16 ? 1 : 0;  // log2(16-byte copies per row of a pair)
@@ -756,18 +987,20 @@ __device__ __forceinline__ void col_fetch(const typename Cplx<T>::type* __restri
       constexpr int NB = H / BH;             // boxes per pair
       constexpr uint32_t kBoxBytes = BH * 2 * sizeof(C);
       static_assert((SZ * sizeof(C)) % 128 == 0 && kBoxBytes % 128 == 0, "TMA boxes start on 128-byte boundaries");
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) tma_bar_expect(bar, (uint32_t)(np * NB) * kBoxBytes);
+      const int c0 = r0 > 0 ? (r0 - 1) / BH + 1 : 0;
+      const int nb = (r1 < H ? r1 / BH + 1 : NB) - c0;  // boxes per pair of this call
+      if (threadIdx.x < 32 && nb > 0) {
+        if (threadIdx.x == 0) tma_bar_expect(bar, (uint32_t)(np * nb) * kBoxBytes);
         __syncwarp();
         tma_proxy_fence();  // the block's earlier use of the buffers comes before the tile writes
-        for (int b = threadIdx.x; b < np * NB; b += 32) {
-          const int q = b / NB, c = b - q * NB;
+        for (int b = threadIdx.x; b < np * nb; b += 32) {
+          const int q = b / nb, c = c0 + b - q * nb;
           tma_load_3d(zb + ((size_t)q * NBUF * SZ + 2 * BH * c) * sizeof(C), tm, bar,
                       (y0 + 2 * q) * (int)(sizeof(C) / 4), BH * c, fidx);
         }
       }
       // row H: one 16-byte unit (float) or two (double) per pair
-      const int units = 1 << ls;
+      const int units = r1 == H ? 1 << ls : 0;
       for (int u = threadIdx.x; u < units; u += blockDim.x) {
         const int part = u & ((1 << LC) - 1);
         const int q = u >> LC;
@@ -777,33 +1010,50 @@ __device__ __forceinline__ void col_fetch(const typename Cplx<T>::type* __restri
       return;
     }
   }
-  const int units = (H + 1) << ls;
+  const int units = (r1 + 1 - r0) << ls;
   for (int u = threadIdx.x; u < units; u += blockDim.x) {
     const int part = u & ((1 << LC) - 1);
     const int q = (u >> LC) & (np - 1);
-    const int kx = u >> ls;
+    const int kx = r0 + (u >> ls);
     cp_async16(zb + ((size_t)q * NBUF * SZ + 2 * kx) * sizeof(C) + part * 16,
                gb + ((size_t)kx * N + 2 * q) * sizeof(C) + part * 16);
   }
 }
 
 // First-pass load of a packed column pair: Z(x) = xa + i xb completed to a
-// Hermitian column (Z(N - kx) = conj xa + i conj xb), from the raw slots.
-template <typename T, int LOG2N, int R>
+// Hermitian column (Z(N - kx) = conj xa + i conj xb), from the raw slots; rows
+// beyond lim are zero, except (BYROW) those flagged in tl, if it is given.
+template <typename T, int LOG2N, int R, bool BYROW>
 __device__ __forceinline__ void col_first_load(const typename Cplx<T>::type* z, int j,
-                                               typename Cplx<T>::type (&v)[R]) {
+                                               typename Cplx<T>::type (&v)[R], int lim,
+                                               const unsigned char* __restrict__ tl) {
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N, H = N / 2, G = N / R;
 #pragma unroll
   for (int m = 0; m < R; ++m) {
     const int x = j + m * G;
     const int kx = x <= H ? x : N - x;
-    C xa, xb;
-    load_pair(z + 2 * kx, xa, xb);
+    C xa = mkc<C>(0, 0), xb = mkc<C>(0, 0);
+    if (kx <= lim || (BYROW && tl && tl[kx])) load_pair(z + 2 * kx, xa, xb);
     if (x == 0 || x == H) v[m] = mkc<C>(xa.x, xb.x);
     else if (x < H) v[m] = mkc<C>(xa.x - xb.y, xa.y + xb.x);
     else v[m] = mkc<C>(xa.x + xb.y, -xa.y + xb.x);
   }
+}
+
+// Where some row beyond pmax is live, all were fetched: the unflagged ones,
+// unwritten in xh, become zero in the raw slots z of a column pair (by the
+// pair's G threads; the caller's barriers lie around it).  Not in the radix-16
+// theta pass, which is at its register cap: the flags in its load's condition
+// measured 159 us against 174 at N = 4096 (scalars' pass the other way round,
+// 113 against 108; multi-size passes 80 against 67).
+template <typename C>
+__device__ __noinline__ void col_zero_rows(C* z, int j, int G, int pmax, int H, const unsigned char* tl) {
+  for (int kx = pmax + 1 + j; kx <= H; kx += G)
+    if (!tl[kx]) {
+      z[2 * kx].x = z[2 * kx].y = 0;
+      z[2 * kx + 1].x = z[2 * kx + 1].y = 0;
+    }
 }
 
 template <typename T, int LOG2N>
@@ -868,64 +1118,107 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
   const C* __restrict__ tw = reinterpret_cast<const C*>(kp.tw);
   const C* xh = reinterpret_cast<const C*>(a.xh);
   const size_t fstride = (size_t)(H + 1) * N;
-  C v[R];
+  // Rows of xh (xh2): those up to pmax are fetched at once, the others -- zero
+  // and unwritten unless flagged -- once the flags have shown one that is not
+  // (the flags' latency passes while the first rows are on their way).
+  const int pin = a.tl ? kp.pmax : H;
+  auto any_row = [&](const unsigned char* t, bool flag) {
+    bool l = false;
+    for (int p = pin + 1 + (int)threadIdx.x; p <= H; p += blockDim.x) l |= (t[p] != 0) == flag;
+    return l;
+  };
+  auto live_rows = [&](const unsigned char* t) { return any_row(t, true); };
+  auto fetch = [&](const C* f, int buf, int fidx, uint64_t* bar) {
+    col_fetch<T, LOG2N, R, NP, NBUF>(f, y0, buf, smem, np, 0, pin, tm, fidx, bar);
+  };
+  auto fetch_rest = [&](const C* f, int buf, int fidx, uint64_t* bar) {
+    col_fetch<T, LOG2N, R, NP, NBUF>(f, y0, buf, smem, np, pin + 1, H, tm, fidx, bar);
+  };
+  constexpr bool BYROW = R == 16 && CMX == CM_THETA;
+  const unsigned char *tl = nullptr, *tl2 = nullptr;  // flags, where a row beyond pmax is live
+  bool dead = false;                                  // ... and another is not
+  auto zero_rows = [&](int b, const unsigned char* t) {
+    col_zero_rows(gbuf + b * SZ, j, G, pin, H, t);
+  };
+  auto first_load = [&](int b, C (&x)[R]) {
+    col_first_load<T, LOG2N, R, BYROW>(gbuf + b * SZ, j, x, !BYROW && tl ? H : pin, tl);
+  };
 
-  if (cmode == CM_VEL && !a.out1) {
-    // u + i v for the scalar passes, column-pair-major (uv_index): both
-    // fields transformed together, one 16-byte (float) or two 16-byte
-    // (double) stores per thread and row
-    col_fetch<T, LOG2N, R, NP, NBUF>(xh, y0, 0, smem, np, tm, 0, &colbar[0]);
-    col_fetch<T, LOG2N, R, NP, NBUF>(xh + fstride, y0, 1, smem, np, tm, 1, &colbar[0]);
-    commit(0);
-    cp_async_wait<0>();
-    __syncthreads();
-    tile_wait(0, 0);
-    C V[2][R];
-    col_first_load<T, LOG2N, R>(gbuf, j, V[0]);
-    col_first_load<T, LOG2N, R>(gbuf + SZ, j, V[1]);
-    fft_multi<T, LOG2N, R, +1, 2>(V, gbuf, SZ, j, tw);
-    C* o = reinterpret_cast<C*>(a.out0);
+  // A column pair's values of a real N x N field at x are adjacent: one store
+  // (load) of both where the field starts on their alignment (a caller's view
+  // need not).
+  auto is_wide = [](const void* f) { return (reinterpret_cast<uintptr_t>(f) & (sizeof(C) - 1)) == 0; };
+  auto store_real = [&](void* f, const C (&x)[R]) {
+    T* o = reinterpret_cast<T*>(f) + ya;
+    const bool wide = is_wide(f);
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      const int x = j + m * G;
-      // V[f][m] = f(x, ya) + i f(x, ya + 1) for f = u, v
-      store_pair(o + uv_index(N, x, ya), mkc<C>(V[0][m].x, V[1][m].x), mkc<C>(V[0][m].y, V[1][m].y));
+      T* q = o + (size_t)(j + m * G) * N;
+      if (wide) {
+        *reinterpret_cast<C*>(q) = x[m];
+      } else {
+        q[0] = x[m].x;
+        q[1] = x[m].y;
+      }
     }
-    return;
-  }
+  };
+  auto load_real = [&](const void* f, int m, bool wide) {
+    const T* q = reinterpret_cast<const T*>(f) + (size_t)(j + m * G) * N + ya;
+    return wide ? *reinterpret_cast<const C*>(q) : mkc<C>(q[0], q[1]);
+  };
+
   if (cmode == CM_VEL || cmode == CM_PHYS1) {
-    const int nf = cmode == CM_VEL ? 2 : 1;
-    for (int f = 0; f < nf; ++f) col_fetch<T, LOG2N, R, NP, NBUF>(xh + f * fstride, y0, f, smem, np, tm, f, &colbar[0]);
+    constexpr int NF = CMX == CM_PHYS1 ? 1 : 2;
+    const int nf = cmode == CM_PHYS1 ? 1 : 2;
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (f < nf) fetch(xh + f * fstride, f, f, &colbar[0]);
+    if (a.tl && __syncthreads_or(live_rows(a.tl))) {
+      tl = a.tl;
+      dead = __syncthreads_or(any_row(tl, false));
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        if (f < nf) fetch_rest(xh + f * fstride, f, f, &colbar[0]);
+    }
     commit(0);
     cp_async_wait<0>();
     __syncthreads();
     tile_wait(0, 0);
-    for (int f = 0; f < nf; ++f) {
-      C* b = gbuf + f * SZ;
-      col_first_load<T, LOG2N, R>(b, j, v);
-      fft_group<T, LOG2N, R, +1>(v, b, j, tw);
-      // v[m] = f(x, ya) + i f(x, ya+1), x = j + m G
-      if (cmode == CM_PHYS1 || a.out1) {
-        T* o = reinterpret_cast<T*>(f == 0 ? a.out0 : a.out1);
-#pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const size_t x = j + m * G;
-          o[x * N + ya] = v[m].x;
-          o[x * N + ya + 1] = v[m].y;
-        }
+    if (dead) {
+      for (int f = 0; f < nf; ++f) zero_rows(f, tl);
+      __syncthreads();
+    }
+    if constexpr (CMX != CM_VEL) {
+      if (cmode == CM_PHYS1) {
+        C V[1][R];
+        first_load(0, V[0]);
+        fft_multi<T, LOG2N, R, +1, 1>(V, gbuf, SZ, j, tw);
+        store_real(a.out0, V[0]);
+        return;
+      }
+    }
+    if constexpr (CMX != CM_PHYS1) {
+      C V[2][R];
+      first_load(0, V[0]);
+      first_load(1, V[1]);
+      fft_multi<T, LOG2N, R, +1, 2>(V, gbuf, SZ, j, tw);
+      // V[f][m] = f(x, ya) + i f(x, ya + 1) for f = u, v
+      if (a.out1) {
+        store_real(a.out0, V[0]);
+        store_real(a.out1, V[1]);
       } else {
-        T* o = reinterpret_cast<T*>(a.out0);  // complex u + i v output
+        // u + i v for the scalar passes, column-pair-major (uv_index): one
+        // 16-byte (float) or two 16-byte (double) stores per thread and row
+        C* o = reinterpret_cast<C*>(a.out0);
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const size_t x = j + m * G;
-          o[2 * (x * N + ya) + f] = v[m].x;
-          o[2 * (x * N + ya + 1) + f] = v[m].y;
-        }
+        for (int m = 0; m < R; ++m)
+          store_pair(o + uv_index(N, j + m * G, ya), mkc<C>(V[0][m].x, V[1][m].x), mkc<C>(V[0][m].y, V[1][m].y));
       }
     }
     return;
   }
 
+  if constexpr (CMX != CM_VEL && CMX != CM_PHYS1) {
   // CM_THETA: the four fields (u, theta_x, v, theta_y) transformed together
   // (NBUF = 4) or in two rounds of two (NBUF = 2); CM_SCAL: one round
   // (s_x, s_y) with (u, v) read from global; CM_FWD: forward transform only.
@@ -940,33 +1233,51 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     const C* xb = cmode == CM_SCALV ? reinterpret_cast<const C*>(a.xh2) : xh;
     const int fb0s = cmode == CM_SCALV ? 0 : fb0, fb1s = cmode == CM_SCALV ? 1 : fb1;
     // (tm is null in CM_SCALV, so the tile fields are always fields of xh)
-    col_fetch<T, LOG2N, R, NP, NBUF>(xh + fa0 * fstride, y0, 0, smem, np, tm, fa0, &colbar[0]);
-    col_fetch<T, LOG2N, R, NP, NBUF>(xb + fb0s * fstride, y0, 1, smem, np, tm, fb0s, &colbar[0]);
-    if (NBUF == 4 && nround == 2) {
-      col_fetch<T, LOG2N, R, NP, NBUF>(xh + fa1 * fstride, y0, 2, smem, np, tm, fa1, &colbar[0]);
-      col_fetch<T, LOG2N, R, NP, NBUF>(xb + fb1s * fstride, y0, 3, smem, np, tm, fb1s, &colbar[0]);
+    const bool two = NBUF == 4 && nround == 2;
+    fetch(xh + fa0 * fstride, 0, fa0, &colbar[0]);
+    fetch(xb + fb0s * fstride, 1, fb0s, &colbar[0]);
+    if (two) {
+      fetch(xh + fa1 * fstride, 2, fa1, &colbar[0]);
+      fetch(xb + fb1s * fstride, 3, fb1s, &colbar[0]);
+    }
+    if (a.tl) {
+      bool live = live_rows(a.tl);
+      if (cmode == CM_SCALV) live |= live_rows(a.tl2);
+      if (__syncthreads_or(live)) {
+        tl = a.tl;
+        tl2 = cmode == CM_SCALV ? a.tl2 : a.tl;
+        if (!BYROW) dead = __syncthreads_or(any_row(tl, false) || any_row(tl2, false));
+        fetch_rest(xh + fa0 * fstride, 0, fa0, &colbar[0]);
+        fetch_rest(xb + fb0s * fstride, 1, fb0s, &colbar[0]);
+        if (two) {
+          fetch_rest(xh + fa1 * fstride, 2, fa1, &colbar[0]);
+          fetch_rest(xb + fb1s * fstride, 3, fb1s, &colbar[0]);
+        }
+      }
     }
     commit(0);
     if (NBUF == 3 && nround == 2) {  // round 2's first field lands in the third buffer during round 1
-      col_fetch<T, LOG2N, R, NP, NBUF>(xh + fa1 * fstride, y0, 2, smem, np, tm, fa1, &colbar[1]);
+      fetch(xh + fa1 * fstride, 2, fa1, &colbar[1]);
+      if (tl) fetch_rest(xh + fa1 * fstride, 2, fa1, &colbar[1]);
       commit(1);
     }
   }
   if (cmode == CM_FWD) {
-    const T* f = reinterpret_cast<const T*>(a.in_real);
+    const bool wide = is_wide(a.in_real);
 #pragma unroll
-    for (int m = 0; m < R; ++m) {
-      const size_t x = j + m * G;
-      W[m] = mkc<C>(f[x * N + ya], f[x * N + ya + 1]);
-    }
+    for (int m = 0; m < R; ++m) W[m] = load_real(a.in_real, m, wide);
   }
   if (NBUF == 4 && nround == 2) {
     cp_async_wait<0>();
     __syncthreads();
     tile_wait(0, 0);
+    if (dead) {
+      for (int f = 0; f < 4; ++f) zero_rows(f, (f & 1) ? tl2 : tl);
+      __syncthreads();
+    }
     C V[4][R];
 #pragma unroll
-    for (int f = 0; f < 4; ++f) col_first_load<T, LOG2N, R>(gbuf + f * SZ, j, V[f]);
+    for (int f = 0; f < 4; ++f) first_load(f, V[f]);
     fft_multi<T, LOG2N, R, +1, 4>(V, gbuf, SZ, j, tw);
     // J = u theta_x + v theta_y for columns a (real parts) and b (imaginary)
     // (CM_SCALV: u s_x + v s_y)
@@ -982,20 +1293,20 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
         store_pair(o + uv_index(N, j + m * G, ya), mkc<C>(V[0][m].x, V[2][m].x), mkc<C>(V[0][m].y, V[2][m].y));
     }
     if (a.in_real) {  // physical-space source: J - src
-      const T* f = reinterpret_cast<const T*>(a.in_real);
+      const bool wide = is_wide(a.in_real);
 #pragma unroll
-      for (int m = 0; m < R; ++m) {
-        const size_t x = j + m * G;
-        W[m].x -= f[x * N + ya];
-        W[m].y -= f[x * N + ya + 1];
-      }
+      for (int m = 0; m < R; ++m) W[m] = csub(W[m], load_real(a.in_real, m, wide));
     }
   } else {
     for (int rd = 0; rd < nround; ++rd) {
       if (rd == 1) {
         __syncthreads();  // round-1 buffers free
-        if (NBUF != 3) col_fetch<T, LOG2N, R, NP, NBUF>(xh + fa1 * fstride, y0, 0, smem, np, tm, fa1, &colbar[0]);
-        col_fetch<T, LOG2N, R, NP, NBUF>(xh + fb1 * fstride, y0, NBUF == 3 ? 0 : 1, smem, np, tm, fb1, &colbar[0]);
+        if (NBUF != 3) fetch(xh + fa1 * fstride, 0, fa1, &colbar[0]);
+        fetch(xh + fb1 * fstride, NBUF == 3 ? 0 : 1, fb1, &colbar[0]);
+        if (tl) {
+          if (NBUF != 3) fetch_rest(xh + fa1 * fstride, 0, fa1, &colbar[0]);
+          fetch_rest(xh + fb1 * fstride, NBUF == 3 ? 0 : 1, fb1, &colbar[0]);
+        }
         commit(0);  // the second phase of mbarrier 0
       }
       if (NBUF == 3 && rd == 0 && nround == 2) cp_async_wait<1>();  // the third buffer's copies may still fly
@@ -1003,13 +1314,16 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
       __syncthreads();
       tile_wait(0, (uint32_t)rd);
       if (NBUF == 3 && rd == 1) tile_wait(1, 0);
+      if (dead) {
+        zero_rows(NBUF == 3 && rd == 1 ? 2 : 0, tl);
+        zero_rows(NBUF == 3 && rd == 1 ? 0 : 1, tl);
+        __syncthreads();
+      }
       C V[2][R];
       // buffers of the round's two fields; the transforms exchange through
       // buffers 0 and 1 (fft_multi synchronises before its first write)
-      const C* b0 = (NBUF == 3 && rd == 1) ? gbuf + 2 * SZ : gbuf;
-      const C* b1 = (NBUF == 3 && rd == 1) ? gbuf : gbuf + SZ;
-      col_first_load<T, LOG2N, R>(b0, j, V[0]);
-      col_first_load<T, LOG2N, R>(b1, j, V[1]);
+      first_load(NBUF == 3 && rd == 1 ? 2 : 0, V[0]);
+      first_load(NBUF == 3 && rd == 1 ? 0 : 1, V[1]);
       fft_multi<T, LOG2N, R, +1, 2>(V, gbuf, SZ, j, tw);
       if (cmode == CM_THETA) {
 #pragma unroll
@@ -1033,13 +1347,9 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     }
   }
   if (!(NBUF == 4 && nround == 2) && cmode == CM_THETA && a.in_real) {  // physical-space source: J - src
-    const T* f = reinterpret_cast<const T*>(a.in_real);
+    const bool wide = is_wide(a.in_real);
 #pragma unroll
-    for (int m = 0; m < R; ++m) {
-      const size_t x = j + m * G;
-      W[m].x -= f[x * N + ya];
-      W[m].y -= f[x * N + ya + 1];
-    }
+    for (int m = 0; m < R; ++m) W[m] = csub(W[m], load_real(a.in_real, m, wide));
   }
   // forward DFT along x of Ja + i Jb
   C* bufX = gbuf;
@@ -1048,10 +1358,11 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
 #pragma unroll
   for (int m = 0; m < R; ++m) bufX[j + m * G] = W[m];
   __syncthreads();
+  // (the rows beyond the band are discarded by the mask: not written)
   // split: Ja(kx) = (W(kx) + conj W(-kx))/2, Jb(kx) = -i (W(kx) - conj W(-kx))/2
   C* jh = reinterpret_cast<C*>(a.jh);
   const int lnp = 31 - __clz(np);  // np is a power of two
-  const int total = (H + 1) << lnp;
+  const int total = ((cmode == CM_FWD ? H : kp.pmax) + 1) << lnp;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
     const int kx = idx >> lnp;
     const int q = idx & (np - 1);
@@ -1062,6 +1373,7 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     const C d = mkc<C>(wk.x - wm.x, wk.y + wm.y);
     const C jb = mkc<C>((T)0.5 * d.y, (T)-0.5 * d.x);
     store_pair(jh + (size_t)kx * N + y0 + 2 * q, ja, jb);
+  }
   }
 }
 

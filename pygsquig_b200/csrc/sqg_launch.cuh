@@ -29,7 +29,7 @@ namespace sqg {
 template <typename T, int L>
 constexpr int col_radix() { return (sizeof(T) == 4 && L >= 11) ? 16 : 8; }
 template <typename T, int L>
-constexpr int row_radix() { return (L >= 7 && L <= 11) ? 4 : 8; }
+constexpr int row_radix() { return (L >= 4 && L <= 11) ? 4 : 8; }
 // The last stage of a step (no inverse transforms) uses the same radix, so
 // that a step and a replayed multistep step round identically.
 template <typename T, int L>
@@ -194,24 +194,26 @@ template <typename T> int multi_col_tiles(int log2n);
 // size of the CTAs change.
 // The row and column passes are launched with programmatic dependent launch
 // (pdl.cuh): the next pass's launch overlaps the tail of the current one.
-// The stage passes of theta and of the scalars run instances compiled for
-// their modes alone (RowInst: N = 4096 FP32 theta stage pass 290 -> 282 us,
-// scalar stage pass 193 -> 184 us) and, at N >= 2048, for their stage too
-// (theta 282 -> 268 us, scalars 184 -> 172 us);
-// the other row passes run the instance that reads its modes from the
-// arguments.
+// Every pass runs an instance compiled for its modes alone (RowInst): the code
+// a block fetches and the registers are those of its kind (stage passes at
+// N = 4096 FP32 290 -> 282 us, scalars 193 -> 184; the transforms of a field
+// with the modes read from the arguments took 158 us against 147 at N = 2048),
+// and at N >= 2048 the stage passes one per stage (theta 282 -> 268 us,
+// scalars 184 -> 172).
 template <typename T, int L>
 constexpr bool row_stage_insts() { return L >= 11; }
 constexpr int row_inst(int rmode, int fmode) {
   if (rmode == RM_P1)
-    return fmode == FM_THETA ? RI_THETA_P1 : (fmode == FM_SCAL ? RI_SCAL_P1 : (fmode == FM_VEL ? RI_VEL_P1 : RI_ANY));
-  return rmode != RM_STAGE ? RI_ANY : (fmode == FM_THETA ? RI_THETA_STAGE : (fmode == FM_SCAL ? RI_SCAL_STAGE : RI_ANY));
+    return fmode == FM_THETA ? RI_THETA_P1 : (fmode == FM_SCAL ? RI_SCAL_P1 : (fmode == FM_VEL ? RI_VEL_P1 : RI_PHYS_P1));
+  if (rmode == RM_RHS) return RI_RHS;
+  if (rmode == RM_SPEC) return RI_SPEC;
+  return fmode == FM_THETA ? RI_THETA_STAGE : RI_SCAL_STAGE;
 }
 template <typename T, int L, int RI>
 cudaError_t launch_row_i(const KP& kp, const RowArgs& a, cudaStream_t st) {
   constexpr int N = 1 << L, RPC = rows_per_cta<T, L>();
-  if constexpr (ri_stage(RI) == 0 && ri_rmode(RI) != RM_P1) {
-    if (a.rmode == RM_STAGE && !a.do_p1) {  // last stage: its own radix, the compiled launch shape
+  if constexpr (RI == RI_THETA_STAGE || RI == RI_SCAL_STAGE) {
+    if (!a.do_p1) {  // last stage: its own radix, the compiled launch shape
       constexpr int RPCX = rowx_rpc<T, L>();
       RowArgs ax = a;
       ax.rpc = 0;
@@ -249,14 +251,13 @@ cudaError_t launch_row_t(const KP& kp, const RowArgs& a, cudaStream_t st) {
     case RI_THETA_P1: return launch_row_i<T, L, RI_THETA_P1>(kp, a, st);
     case RI_SCAL_P1: return launch_row_i<T, L, RI_SCAL_P1>(kp, a, st);
     case RI_VEL_P1: return launch_row_i<T, L, RI_VEL_P1>(kp, a, st);
-    default: return launch_row_i<T, L, RI_ANY>(kp, a, st);
+    case RI_PHYS_P1: return launch_row_i<T, L, RI_PHYS_P1>(kp, a, st);
+    case RI_RHS: return launch_row_i<T, L, RI_RHS>(kp, a, st);
+    default: return launch_row_i<T, L, RI_SPEC>(kp, a, st);
   }
 }
-// Column passes of theta and of the scalars run instances compiled for their
-// mode alone (fewer registers live, fewer spills: N = 4096 FP32 theta column
-// pass 212 -> 204 us, scalar column pass 149 -> 134 us); the other modes run
-// the instance that chooses the mode at run time (an instance for the
-// velocity pass alone was slower, 90 -> 92 us).
+// Column passes likewise run one instance per mode (N = 4096 FP32 theta column
+// pass 212 -> 204 us, scalar column pass 149 -> 134 us).
 // Field buffers per column pair of a mode instance: theta's two-round pass at
 // N = 4096 keeps a third, which receives round 2's first field during round 1
 // (FP32 205 -> 197 us, FP64 532 -> 518 us).
@@ -286,8 +287,10 @@ cudaError_t launch_col_t(const KP& kp, const ColArgs& a, cudaStream_t st, bool r
   const int np = a.np > 0 ? a.np : NP;
   const int grid = ring_only ? 1 : N / (2 * np) + (a.ring_cta ? 1 : 0);
   if (a.cmode == CM_THETA) return launch_col_m<T, L, CM_THETA>(kp, a, st, grid, np, tm);
-  if (a.cmode == CM_SCAL && !a.ring_cta) return launch_col_m<T, L, CM_SCAL>(kp, a, st, grid, np, tm);
-  return launch_col_m<T, L, -1>(kp, a, st, grid, np, tm);
+  if (a.cmode == CM_SCAL) return launch_col_m<T, L, CM_SCAL>(kp, a, st, grid, np, tm);
+  if (a.cmode == CM_VEL) return launch_col_m<T, L, CM_VEL>(kp, a, st, grid, np, tm);
+  if (a.cmode == CM_PHYS1) return launch_col_m<T, L, CM_PHYS1>(kp, a, st, grid, np, tm);
+  return launch_col_m<T, L, CM_FWD>(kp, a, st, grid, np, tm);
 }
 template <typename T, int L>
 cudaError_t shape_max_t(int* rpc, int* np) {
@@ -300,7 +303,7 @@ cudaError_t set_row_attrs_i() {
   constexpr int RPC = rows_per_cta<T, L>();
   cudaError_t e = cudaFuncSetAttribute(k_row<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>(), RI>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T, L>());
-  if constexpr (ri_stage(RI) == 0 && ri_rmode(RI) != RM_P1) {  // the last-stage kernel: the stage instances
+  if constexpr (RI == RI_THETA_STAGE || RI == RI_SCAL_STAGE) {  // the last-stage kernel: the stage instances
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_row<T, L, rowx_radix<T, L>(), rowx_rpc<T, L>(), rowx_depth<T, L>(), 0, RI>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowx_smem<T, L>(rowx_depth<T, L>()));
@@ -315,12 +318,14 @@ cudaError_t set_row_stage_attrs_i() {
   if (e == cudaSuccess) e = set_row_attrs_i<T, L, RI0 + 3>();
   return e;
 }
+template <typename T, int L, int CMX>
+cudaError_t set_col_attrs_m() {
+  return cudaFuncSetAttribute(k_col<T, L, col_radix<T, L>(), pairs_per_cta<T, L>(), col_nbuf_m<T, L, CMX>(), CMX>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem_m<T, L, CMX>());
+}
 template <typename T, int L>
 cudaError_t set_attrs_t() {
-  constexpr int NP = pairs_per_cta<T, L>();
-  cudaError_t e = set_row_attrs_i<T, L, RI_ANY>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_THETA_STAGE>();
+  cudaError_t e = set_row_attrs_i<T, L, RI_THETA_STAGE>();
   if (e != cudaSuccess) return e;
   e = set_row_attrs_i<T, L, RI_SCAL_STAGE>();
   if (e != cudaSuccess) return e;
@@ -330,20 +335,24 @@ cudaError_t set_attrs_t() {
   if (e != cudaSuccess) return e;
   e = set_row_attrs_i<T, L, RI_VEL_P1>();
   if (e != cudaSuccess) return e;
+  e = set_row_attrs_i<T, L, RI_PHYS_P1>();
+  if (e != cudaSuccess) return e;
+  e = set_row_attrs_i<T, L, RI_RHS>();
+  if (e != cudaSuccess) return e;
+  e = set_row_attrs_i<T, L, RI_SPEC>();
+  if (e != cudaSuccess) return e;
   if constexpr (row_stage_insts<T, L>()) {
     e = set_row_stage_attrs_i<T, L, RI_THETA_S1>();
     if (e != cudaSuccess) return e;
     e = set_row_stage_attrs_i<T, L, RI_SCAL_S1>();
     if (e != cudaSuccess) return e;
   }
-  e = cudaFuncSetAttribute(k_col<T, L, col_radix<T, L>(), NP, col_nbuf_m<T, L, CM_THETA>(), CM_THETA>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem_m<T, L, CM_THETA>());
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_col<T, L, col_radix<T, L>(), NP, col_nbuf<T, L>(), CM_SCAL>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem<T, L>());
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_col<T, L, col_radix<T, L>(), NP, col_nbuf<T, L>()>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem<T, L>());
+  e = set_col_attrs_m<T, L, CM_THETA>();
+  if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_SCAL>();
+  if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_VEL>();
+  if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_PHYS1>();
+  if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_FWD>();
+  return e;
 }
 
 template <typename T, int L>
