@@ -59,7 +59,7 @@ constexpr int kC = 64;
 constexpr int kSlabRows = kTileM + 2;        // pixels of one input-row slab
 constexpr int kSlabBytes = kSlabRows * 128;  // 16640 B loaded per slab
 constexpr int kSlabStride = 17 * 1024;       // slabs start on 1024-byte boundaries
-constexpr int kStages = 6;                   // slabs in flight (two tiles)
+constexpr int kStages = 5;                   // slabs in flight (a tile and two thirds)
 constexpr int kBBytes = kC * kC * 2;         // 8 KB per tap
 constexpr int kStageTile = kTileM * 128;     // 16 KB staging tile (128 pixels x 64 BF16)
 constexpr int kThreads = 320;
@@ -107,8 +107,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
-// the staging tiles may be rewritten once the stores issued so far have read them
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+// a pair of staging tiles may be rewritten once the stores before the last group have read it
+__device__ __forceinline__ void bulk_wait_read_prev() { asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 // generic-proxy shared-memory writes become visible to the TMA (async proxy)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
@@ -207,9 +207,8 @@ k_conv64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CU
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sB = base;                                   // 9 x 8 KB weights
   unsigned char* sA = sB + 9 * kBBytes;                       // kStages row slabs
-  unsigned char* sO = sA + kStages * kSlabStride;             // staging: halo'd output tile
-  unsigned char* sZ = sO + kStageTile;                        // staging: pre-activation tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sZ + kStageTile);
+  unsigned char* sS = sA + kStages * kSlabStride;             // staging, two pairs: output tile, pre-activation tile
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sS + 4 * kStageTile);
   uint64_t* full = bars;                 // [kStages]
   uint64_t* empty = bars + kStages;      // [kStages]
   uint64_t* acc_full = bars + 2 * kStages;   // [2]
@@ -320,30 +319,42 @@ k_conv64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CU
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tcount) {
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
-      const int bad = mbar_wait(&acc_full[acc], aph) ? 0 : 1;
-      if (leader) bulk_wait_read_all();  // the staging tiles are free again
-      if (epi_sync_or(bad)) { ok = false; break; }
-      tc_fence_after();
-      float v[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = bz[i];
-      const uint32_t taddr = tmem + acc * 256 + c0 + ((uint32_t)(quarter * 32) << 16);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        uint32_t r[32];
-        TC_LD32(taddr + 64 * k, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r[i]);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[acc]);
       const int xt = tile % tiles_per_row;
       const int rowi = tile / tiles_per_row;
       const int y = rowi % a.H, b = rowi / a.H;
       const int x = xt * kTileM + row;
       const size_t pix = ((size_t)b * a.H + y) * a.W + x;
+      // the pre-activations of the layer below, requested ahead of the wait
+      uint4 zq[4];
+      if (a.mode == CLOSURE_EPI_DGRAD) {
+        const uint4* zsrc = reinterpret_cast<const uint4*>(a.zprev + pix * kC + c0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) zq[i] = zsrc[i];
+      }
+      const int bad = mbar_wait(&acc_full[acc], aph) ? 0 : 1;
+      if (leader) bulk_wait_read_prev();  // this tile's pair of staging tiles is free again
+      if (epi_sync_or(bad)) { ok = false; break; }
+      tc_fence_after();
+      unsigned char* sO = sS + acc * 2 * kStageTile;
+      unsigned char* sZ = sO + kStageTile;
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = bz[i];
+      const uint32_t taddr = tmem + acc * 256 + c0 + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+      for (int k = 0; k < 4; k += 2) {  // two accumulators per wait
+        uint32_t r0[32], r1[32];
+        TC_LD32(taddr + 64 * k, r0);
+        TC_LD32(taddr + 64 * k + 64, r1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r0[i]);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(r1[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[acc]);
       if (a.mode == CLOSURE_EPI_LIN) {
         float4* o = reinterpret_cast<float4*>(a.out_f32 + pix * kC + c0);
 #pragma unroll
@@ -356,22 +367,18 @@ k_conv64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CU
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const __nv_bfloat162 zb = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-          const float2 zr = __bfloat1622float2(zb);  // the stored pre-activation
           reinterpret_cast<__nv_bfloat162*>(zp)[i] = zb;
-          reinterpret_cast<__nv_bfloat162*>(packed)[i] = __floats2bfloat162_rn(gelu(zr.x), gelu(zr.y));
+          const float2 av = gelu2(__bfloat1622float2(zb));  // of the stored pre-activation
+          reinterpret_cast<__nv_bfloat162*>(packed)[i] = __floats2bfloat162_rn(av.x, av.y);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(sZ + sw128_off(row, (c0 >> 3) + i)) = zp[i];
       } else {  // DGRAD
-        const uint4* zsrc = reinterpret_cast<const uint4*>(a.zprev + pix * kC + c0);
-        uint4 zq[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) zq[i] = zsrc[i];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float2 z = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(zq)[i]);
-          reinterpret_cast<__nv_bfloat162*>(packed)[i] =
-              __floats2bfloat162_rn(v[2 * i] * gelu_grad(z.x), v[2 * i + 1] * gelu_grad(z.y));
+          const float2 g = __fmul2_rn(make_float2(v[2 * i], v[2 * i + 1]), gelu_grad2(z));
+          reinterpret_cast<__nv_bfloat162*>(packed)[i] = __floats2bfloat162_rn(g.x, g.y);
         }
       }
 #pragma unroll
@@ -554,15 +561,18 @@ k_wgrad64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ C
   }
 }
 
-// dW[t][co][ci] = sum over CTAs of partials[cta][t/2][(t%2)*64 + ci][co]
+// dW[t][co][ci] = sum over CTAs of partials[cta][t/2][(t%2)*64 + ci][co].  Threads
+// run along co, as the partials do (along ci each load of a warp took 32
+// sectors: 23 us).
 __global__ void k_wgrad_reduce(const float* __restrict__ partials, int nparts, float* __restrict__ dw) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;  // over 9 * 64 * 64
   if (idx >= 9 * 64 * 64) return;
-  const int t = idx / 4096, co = (idx / 64) % 64, ci = idx % 64;
-  const size_t off = ((size_t)(t / 2) * 128 + (t % 2) * 64 + ci) * 64 + co;
+  const int t = idx / 4096, ci = (idx / 64) % 64, co = idx % 64;
+  const float* p = partials + ((size_t)(t / 2) * 128 + (t % 2) * 64 + ci) * 64 + co;
   float s = 0.f;
-  for (int c = 0; c < nparts; ++c) s += partials[(size_t)c * 5 * 128 * 64 + off];
-  dw[idx] = s;
+#pragma unroll 16
+  for (int c = 0; c < nparts; ++c) s += p[(size_t)c * 5 * 128 * 64];
+  dw[t * 4096 + co * 64 + ci] = s;
 }
 
 // ---- host: tensor maps through the driver entry point -------------------------
@@ -595,7 +605,7 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint32_t box_rows)
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr size_t kSmemBytes = 1024 + 9 * kBBytes + kStages * kSlabStride + 2 * kStageTile + 256;
+constexpr size_t kSmemBytes = 1024 + 9 * kBBytes + kStages * kSlabStride + 4 * kStageTile + 256;
 
 }  // namespace
 
