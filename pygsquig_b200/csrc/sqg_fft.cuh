@@ -276,6 +276,9 @@ template <> struct FftElem<Dual> {
   }
 };
 
+template <typename T, int LOG2N, int R>
+__host__ __device__ constexpr bool fft_tw2() { return sizeof(T) == 4 && R == 8 && LOG2N == 11; }
+
 template <typename T, int LOG2N, int R, int DIR, int NE, typename E>
 __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, int j,
                                           const typename Cplx<T>::type* __restrict__ tw) {
@@ -299,8 +302,17 @@ __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, i
   // pass's root is loaded one pass ahead so the load's latency (the table is
   // often not L1-resident next to large shared-memory buffers) overlaps the
   // butterflies and exchange of the pass before.
-  auto root = [&](int pp, int lpp) -> C { return tw[((j & (pp - 1)) << (LOG2N - lpp - LR)) & (N - 1)]; };
-  C w_next = REM != 0 ? root(1 << REM, REM) : C{};
+  // (TW2: w and w^3 from the table instead of w alone: powers of w carry its
+  // rounding r-fold, and the radix-8 row pass that serves N = 2048 instead of a
+  // radix-4 one is to be no further from exact: at w, w^3 the squared errors of
+  // its twiddles sum to 12 units over its passes, to 17.5 in radix 4, to 52 from
+  // w alone.)
+  constexpr bool TW2 = fft_tw2<T, LOG2N, R>();
+  auto root = [&](int pp, int lpp, int e) -> C {
+    return tw[((e * (j & (pp - 1))) << (LOG2N - lpp - LR)) & (N - 1)];
+  };
+  C w_next = REM != 0 ? root(1 << REM, REM, 1) : C{};
+  C w3_next = REM != 0 && TW2 ? root(1 << REM, REM, 3) : C{};
   int p = 1;
   if (REM != 0) {
     constexpr int RP = 1 << REM;
@@ -340,8 +352,11 @@ __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, i
 #pragma unroll 1
   for (int pass = 0; pass < NPR; ++pass) {
     const int k = j & (p - 1);
-    const C w_cur = w_next;
-    if (pass + 1 < NPR) w_next = root(p * R, lp + LR);
+    const C w_cur = w_next, w3_cur = w3_next;
+    if (pass + 1 < NPR) {
+      w_next = root(p * R, lp + LR, 1);
+      if (TW2) w3_next = root(p * R, lp + LR, 3);
+    }
     if (p > 1) {
       // w^r for r = 1..R-1 from one table load w = exp(-+2 pi i k / (p R)):
       // powers by complex products (at most three chained roundings)
@@ -349,10 +364,10 @@ __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, i
       C wp[R];
       wp[1] = w1;
       wp[2] = cmul(w1, w1);
-      wp[3] = cmul(wp[2], w1);
+      wp[3] = TW2 ? w3_cur : cmul(wp[2], w1);
       if constexpr (R >= 8) {
-        wp[4] = cmul(wp[2], wp[2]);
-        wp[5] = cmul(wp[4], w1);
+        wp[4] = TW2 ? cmul(wp[3], w1) : cmul(wp[2], wp[2]);
+        wp[5] = TW2 ? cmul(wp[3], wp[2]) : cmul(wp[4], w1);
         wp[6] = cmul(wp[3], wp[3]);
         wp[7] = cmul(wp[4], wp[3]);
       }

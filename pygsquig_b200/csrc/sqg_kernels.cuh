@@ -367,12 +367,26 @@ __host__ __device__ constexpr int fs_kind(int fs, int f) {
   return fs == FS_ID ? FK_ID : (fs == FS_GRAD ? FK_DX + f : f);
 }
 
+// |k|^-alpha of a thread's R modes (row_fields' frac).
+template <typename T, int LOG2N, int R>
+__device__ __forceinline__ void row_frac(const KP& kp, int j, int p, T (&frac)[R]) {
+  constexpr int N = 1 << LOG2N;
+  const T kx = wavenumber_mt<T>(kp, p < N / 2 ? p : p - N);
+  T k2[R];
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    const T ky = wavenumber_mt<T>(kp, RowElem<N, R>::mode(j, m));
+    k2[m] = kx * kx + ky * ky;
+  }
+  inv_frac<T, R>(k2, (T)kp.alpha, kp.akind, frac);
+}
+
 // The fields of set FS of the row pair's mode: form their spectra from
 // theta_{s+1} at (p, iy) / (N-p, N-iy), transform them together along y and
 // write xh[f0 + f][p][:].  SRC: also the mean-gradient sources (velocity pass).
 template <typename T, int LOG2N, int R, int FS, bool SRC, bool OFF, typename HA>
 __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha, int f0, int j, int p, bool valid,
-                                           typename Cplx<T>::type* wbuf) {
+                                           typename Cplx<T>::type* wbuf, const T (&frac)[R]) {
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N, G = N / R, H = N / 2, XB = spad_size<R>(N);
   constexpr int NF = fs_fields(FS);
@@ -384,16 +398,6 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
   const T dkx = (p == H) ? (T)0 : kx;
   const T nkx = (p == H) ? kx : (T)0;
   C V[NF][R];
-  T frac[R];
-  if constexpr (uv) {
-    T k2[R];
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      const T ky = wavenumber_mt<T>(kp, E::mode(j, m));
-      k2[m] = kx * kx + ky * ky;
-    }
-    inv_frac<T, R>(k2, (T)kp.alpha, kp.akind, frac);
-  }
 #pragma unroll
   for (int m = 0; m < R; ++m) {
     const int iy = j + m * G;
@@ -495,6 +499,9 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   bool bad = false, skip_p1 = false;
   __shared__ bool warp_out[32];  // RM_P1: a warp saw a mode outside the band
 
+  // |k|^-alpha ahead of the transforms (stage passes), or as they begin
+  constexpr bool FRAC0 = R == 4 && !BATCH && LOG2N <= 9 && ri_rmode(RI) == RM_STAGE && ri_fmode(RI) == FM_THETA && NFX > 0;
+  T frac[R];
   C v[R];   // FFT registers
   C t1[R];  // theta_{s+1} (or theta_in) at e1 = (p, iy)
   C t2[R];  // theta_{s+1} at e2 = (pp, N - iy)
@@ -606,17 +613,18 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
       }
     };
     // The radix-4 passes are bound by the latency of their one wave of blocks:
-    // they evaluate the operator for all their elements ahead of the transform
-    // (independent chains, while the loads are under way) and update them
-    // without branches.  The radix-8 passes, short of registers and with more
+    // they evaluate the operator and |k|^-alpha for all their elements ahead of
+    // the transform (independent chains, while the loads are under way) and
+    // update them without branches.  The radix-8 passes, short of registers and with more
     // warps to hide a chain, branch around each element outside the band.
-    constexpr bool HOIST = R == 4 && sizeof(T) == 4 && !BATCH;
+    constexpr bool HOIST = R == 4 && (sizeof(T) == 4 || LOG2N <= 9) && !BATCH;
     constexpr bool FLAT = HOIST || sizeof(T) == 8;
     T fe[HOIST ? R : 1], fe2[HOIST ? R : 1], fl[HOIST ? R : 1];
     if constexpr (HOIST) {
 #pragma unroll
       for (int m = 0; m < R; ++m) linear(m, fe[m], fe2[m], fl[m]);
     }
+    if constexpr (FRAC0) row_frac<T, LOG2N, R>(kp, j, p, frac);
     if (use_j) fft_group<T, LOG2N, R, -1>(v, wbuf, j, tw);
     // v[m] = J^(p, iy) ; J^(pp, N - iy) = conj(v[m])
     if (rmode == RM_SPEC) {
@@ -847,19 +855,20 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   // the batch with u and v also writes the mean-gradient sources).
   static_assert(NFT == 2 || NFT == 4, "row passes with transforms take two or four fields at a time");
   auto fields = [&](auto ha) {
+    if (!FRAC0 && (fmode == FM_THETA || fmode == FM_VEL)) row_frac<T, LOG2N, R>(kp, j, p, frac);
     if (fmode == FM_THETA) {
       if constexpr (NFT == 4) {
-        row_fields<T, LOG2N, R, FS_ALL, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
+        row_fields<T, LOG2N, R, FS_ALL, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf, frac);
       } else {
-        row_fields<T, LOG2N, R, FS_UV, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
-        row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 2, j, p, valid, wbuf);
+        row_fields<T, LOG2N, R, FS_UV, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf, frac);
+        row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 2, j, p, valid, wbuf, frac);
       }
     } else if (fmode == FM_PHYS1) {
-      row_fields<T, LOG2N, R, FS_ID, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_ID, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf, frac);
     } else if (fmode == FM_VEL) {
-      row_fields<T, LOG2N, R, FS_UV, RI == RI_VEL_P1, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_UV, RI == RI_VEL_P1, BATCH>(kp, a, ha, 0, j, p, valid, wbuf, frac);
     } else {
-      row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf);
+      row_fields<T, LOG2N, R, FS_GRAD, false, BATCH>(kp, a, ha, 0, j, p, valid, wbuf, frac);
     }
   };
   if constexpr (nfx_park(NFX)) fields(ha_smem);

@@ -29,7 +29,7 @@ namespace sqg {
 template <typename T, int L>
 constexpr int col_radix() { return (sizeof(T) == 4 && L >= 11) ? 16 : 8; }
 template <typename T, int L>
-constexpr int row_radix() { return (L >= 4 && L <= 11) ? 4 : 8; }
+constexpr int row_radix() { return (L >= 4 && L <= (sizeof(T) == 4 ? 10 : 11)) ? 4 : 8; }
 // The last stage of a step (no inverse transforms) uses the same radix, so
 // that a step and a replayed multistep step round identically.
 template <typename T, int L>
@@ -72,7 +72,7 @@ constexpr int col_nbuf() {
 // stage pass 221 -> 202 us against one field at a time).
 template <typename T, int L>
 constexpr int row_nfx() {
-  if (sizeof(T) == 4 && L == 12) return 6;
+  if (sizeof(T) == 4 && L >= 11) return 6;
   return row_radix<T, L>() != 8 ? 2
          : (size_t)rows_per_cta<T, L>() * 4 * spad_size<row_radix<T, L>()>(1 << L) * sizeof(typename Cplx<T>::type) <=
                    150 * 1024 ? 4 : 2;
@@ -198,10 +198,9 @@ template <typename T> int multi_col_tiles(int log2n);
 // a block fetches and the registers are those of its kind (stage passes at
 // N = 4096 FP32 290 -> 282 us, scalars 193 -> 184; the transforms of a field
 // with the modes read from the arguments took 158 us against 147 at N = 2048),
-// and at N >= 2048 the stage passes one per stage (theta 282 -> 268 us,
-// scalars 184 -> 172).
-template <typename T, int L>
-constexpr bool row_stage_insts() { return L >= 11; }
+// and the stage passes with transforms one per stage (N = 4096 theta 282 -> 268
+// us, scalars 184 -> 172; N = 1024 10 steps FP32 1207 -> 1165 us, 5 steps FP64 1103
+// -> 1056).
 constexpr int row_inst(int rmode, int fmode) {
   if (rmode == RM_P1)
     return fmode == FM_THETA ? RI_THETA_P1 : (fmode == FM_SCAL ? RI_SCAL_P1 : (fmode == FM_VEL ? RI_VEL_P1 : RI_PHYS_P1));
@@ -239,11 +238,9 @@ cudaError_t launch_row_stage_i(const KP& kp, const RowArgs& a, cudaStream_t st) 
 template <typename T, int L>
 cudaError_t launch_row_t(const KP& kp, const RowArgs& a, cudaStream_t st) {
   const int ri = row_inst(a.rmode, a.fmode);
-  if constexpr (row_stage_insts<T, L>()) {
-    if (a.do_p1 && a.stage >= 1 && a.stage <= 4) {
-      if (ri == RI_THETA_STAGE) return launch_row_stage_i<T, L, RI_THETA_S1>(kp, a, st);
-      if (ri == RI_SCAL_STAGE) return launch_row_stage_i<T, L, RI_SCAL_S1>(kp, a, st);
-    }
+  if (a.do_p1 && a.stage >= 1 && a.stage <= 4) {
+    if (ri == RI_THETA_STAGE) return launch_row_stage_i<T, L, RI_THETA_S1>(kp, a, st);
+    if (ri == RI_SCAL_STAGE) return launch_row_stage_i<T, L, RI_SCAL_S1>(kp, a, st);
   }
   switch (ri) {
     case RI_THETA_STAGE: return launch_row_i<T, L, RI_THETA_STAGE>(kp, a, st);
@@ -341,12 +338,10 @@ cudaError_t set_attrs_t() {
   if (e != cudaSuccess) return e;
   e = set_row_attrs_i<T, L, RI_SPEC>();
   if (e != cudaSuccess) return e;
-  if constexpr (row_stage_insts<T, L>()) {
-    e = set_row_stage_attrs_i<T, L, RI_THETA_S1>();
-    if (e != cudaSuccess) return e;
-    e = set_row_stage_attrs_i<T, L, RI_SCAL_S1>();
-    if (e != cudaSuccess) return e;
-  }
+  e = set_row_stage_attrs_i<T, L, RI_THETA_S1>();
+  if (e != cudaSuccess) return e;
+  e = set_row_stage_attrs_i<T, L, RI_SCAL_S1>();
+  if (e != cudaSuccess) return e;
   e = set_col_attrs_m<T, L, CM_THETA>();
   if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_SCAL>();
   if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_VEL>();
