@@ -201,7 +201,6 @@ __device__ __forceinline__ uint32_t sw128_off(int r, int c) { return (uint32_t)r
 __global__ void __launch_bounds__(kThreads, 1)
 k_conv64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CUtensorMap w_map,
          const __grid_constant__ CUtensorMap out_map, const __grid_constant__ CUtensorMap z_map, ConvArgs a) {
-  pdl_wait();  // the previous kernel's output (this layer's input) is visible after this
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // 1024-byte aligned carve-up
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -243,6 +242,9 @@ k_conv64(const __grid_constant__ CUtensorMap act_map, const __grid_constant__ CU
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   bool ok = true;
+  // the previous kernel's output (this layer's input) is visible after this; the
+  // set-up above overlaps that kernel's end (batch 1: 12.6 -> 12.4 us a layer)
+  pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
