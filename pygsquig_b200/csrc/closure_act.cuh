@@ -29,5 +29,5 @@ __device__ __forceinline__ float2 gelu_grad2(float2 z) {
   const float2 h = __fmul2_rn(f2(0.5f), __fadd2_rn(f2(1.0f), t));
   const float2 d = __ffma2_rn(make_float2(-t.x, -t.y), t, f2(1.0f));  // 1 - t^2
   const float2 q = __fmul2_rn(__fmul2_rn(__fmul2_rn(f2(0.5f), z), d), f2(kGeluA));
-  return __ffma2_rn(q, __ffma2_rn(f2(3.0f * kGeluB), z2, f2(1.0f)), h);
+  return __fadd2_rn(h, __fmul2_rn(q, __ffma2_rn(f2(3.0f * kGeluB), z2, f2(1.0f))));
 }
