@@ -277,7 +277,7 @@ template <> struct FftElem<Dual> {
 };
 
 template <typename T, int LOG2N, int R>
-__host__ __device__ constexpr bool fft_tw2() { return sizeof(T) == 4 && R == 8 && LOG2N == 11; }
+__host__ __device__ constexpr bool fft_tw2() { return R == 8 && LOG2N == 11; }
 
 template <typename T, int LOG2N, int R, int DIR, int NE, typename E>
 __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, int j,

@@ -15,21 +15,20 @@ namespace sqg {
 
 // ---- compile-time launch shapes ----
 // Radix of the group FFTs.  Column pass: 16 for float grids with N >= 2048
-// (groups of N/16 threads, one exchange pass fewer, two 256-thread blocks per
-// SM; measured at N = 4096: 370 -> 271 us per launch); row pass: 8 at those
-// sizes (radix 16 with two exchange buffers made the fused stage pass slower,
-// 384 -> 508 us, because its stage update walks 16 prefetched chunks per
-// thread).  Grids with 128 <= N <= 2048: radix-4 row pass (twice the threads
-// per transform at 64 registers in single precision, 128 in double; at
-// N <= 1024 the pass is one wave of blocks bound by each block's latency:
-// FP32 N = 1024 row passes 31 -> 20 us, FP64 52 -> 36 us; N = 2048 step
-// FP32 0.64 -> 0.57 ms, FP64 1.36 -> 1.19 ms; at N = 4096 it was slower,
-// 315 -> 357 us); the column pass stays radix 8 there (radix 4 took
-// 23 -> 30 us at N = 1024 in single precision, 34 -> 39 us in double).
+// (groups of N/16 threads, one exchange pass fewer; N = 4096 370 -> 271 us, N =
+// 2048 4 steps 1447 -> 1417 us), else 8.  Row pass: 8 at N = 4096 (radix 16 made
+// the fused stage pass slower, 384 -> 508 us, radix 4 315 -> 357 us) and, with
+// theta parked (row_nfx), at 2048 (radix 4: N = 2048 stage pass FP32 60 against 42
+// us, FP64 step with two scalars 2.70 against 2.40 ms).  N = 16 to 1024: radix 4
+// (twice the threads per transform at 64 registers in single precision, 128 in
+// double: those passes are one wave of blocks bound by each block's latency;
+// N = 1024 stage pass 19 us, 25 in radix 8; N = 64 FP64 step 80 -> 57 us); the
+// column pass stays radix 8 there (radix 4 took 23 -> 30 us at N = 1024 in single
+// precision, 34 -> 39 us in double).
 template <typename T, int L>
 constexpr int col_radix() { return (sizeof(T) == 4 && L >= 11) ? 16 : 8; }
 template <typename T, int L>
-constexpr int row_radix() { return (L >= 4 && L <= (sizeof(T) == 4 ? 10 : 11)) ? 4 : 8; }
+constexpr int row_radix() { return (L >= 4 && L <= 10) ? 4 : 8; }
 // The last stage of a step (no inverse transforms) uses the same radix, so
 // that a step and a replayed multistep step round identically.
 template <typename T, int L>
@@ -65,14 +64,16 @@ constexpr int col_nbuf() {
 }
 // Fields the row pass transforms together (row_body's NFX): four (one
 // exchange buffer each) when their buffers fit in 150 KB, else two (two
-// rounds); two for a radix-4 or radix-16 row pass.  FP32 at N = 4096 takes
-// two at a time with theta_{s+1} parked in shared memory (NFX = 6) at 64
-// registers, two 512-thread blocks per SM (measured against four fields from
-// registers at one block per SM: theta stage pass 332 -> 289 us; scalar
-// stage pass 221 -> 202 us against one field at a time).
+// rounds); two for a radix-4 or radix-16 row pass.  N = 2048, and FP32 at N =
+// 4096, take two at a time with theta_{s+1} parked in shared memory (NFX = 6) at
+// 64 registers (128 in double), which lets two 512-thread blocks share an SM at
+// 4096 (theta stage pass 332 -> 289 us against four fields from registers) and
+// four (two in double) of 256 at 2048.  FP64 at 4096 has one block per SM either
+// way and does better from registers (step with two scalars 9.66 against 9.75
+// ms).
 template <typename T, int L>
 constexpr int row_nfx() {
-  if (sizeof(T) == 4 && L >= 11) return 6;
+  if (L == 11 || (sizeof(T) == 4 && L == 12)) return 6;
   return row_radix<T, L>() != 8 ? 2
          : (size_t)rows_per_cta<T, L>() * 4 * spad_size<row_radix<T, L>()>(1 << L) * sizeof(typename Cplx<T>::type) <=
                    150 * 1024 ? 4 : 2;
