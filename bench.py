@@ -129,7 +129,8 @@ def pass_bytes(N, w_bytes, n_scalars=0, n_src=0):
       col_scalar    2h + u + i v (f) in, J^ (h) out
       row_scalar    s=1: h, s_n (f), acc out (f), 2h; s=2,3: h, f, 2f, 2h;
                     s=4: h, acc in (f), s_{n+1} out (f); plus its source (h)
-    Ring-mode tables and phases are negligible.
+    Ring-mode tables and phases are negligible.  Every mode counts: where a
+    field is zero outside the dealiasing disk the passes move less.
     """
     h = (N // 2 + 1) * N * 2 * w_bytes
     f = N * N * 2 * w_bytes
