@@ -131,7 +131,8 @@ struct RowArgs {
   void* src_out[4];
   double gx[4], gy[4];
   int rpc;                        // row pairs per CTA (0: the compiled maximum RPC)
-  int st_zero;                    // 1: st_out is read outside the passes (zeros stored outside the band too)
+  int st_zero;                    // 1: st_out is read outside the passes, and a later stage may add a term outside
+                                  // the band (stage 1 stores zeros there, in st_out and acc)
   unsigned char* tl;              // out-of-band flags of the field's row pairs (null: every row takes every mode)
   const unsigned char* tl_src;    // flags of src_h's rows (the theta its velocity came from)
 };
@@ -546,17 +547,34 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
         tile_tail |= t;
       }
     }
+    // Where the zeros outside the band have to be stored.  Stage buffer and
+    // accumulator: once a step, by stage 1 (no later stage touches them unless
+    // the row is flagged by then, and then it writes every mode), when
+    // the stages are separate calls: the caller reads the buffer, and a term
+    // given to a later stage meets the accumulator outside the band.
+    auto zero_out = [&]() -> void* {
+      return rmode == RM_RHS ? a.rhs_out
+             : stage == 4    ? (a.th_out != a.th_n ? a.th_out : nullptr)
+                             : (stage == 1 && a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
+    };
+    auto zero_acc = [&]() -> void* { return rmode == RM_STAGE && stage == 1 && a.st_zero ? a.acc : nullptr; };
+    auto zero_mode = [&](void* z1, void* z2, int m) {
+      if (z1) {
+        *rp.at(z1, m) = mkc<C>(0, 0);
+        if (pair) *rp.mir(z1, m) = mkc<C>(0, 0);
+      }
+      if (z2) {
+        *rp.at(z2, m) = mkc<C>(0, 0);
+        if (pair) *rp.mir(z2, m) = mkc<C>(0, 0);
+      }
+    };
     if (tile_out && !tile_tail && rmode != RM_SPEC) {
       // every mode of the block's rows is zero and stays zero
-      void* z1 = rmode == RM_RHS ? a.rhs_out
-                 : stage == 4    ? (a.th_out != a.th_n ? a.th_out : nullptr)
-                                 : (a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
-      if (z1 && valid) {
+      void* z1 = zero_out();
+      void* z2 = zero_acc();
+      if (valid && (z1 || z2)) {
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-          *rp.at(z1, m) = mkc<C>(0, 0);
-          if (pair) *rp.mir(z1, m) = mkc<C>(0, 0);
-        }
+        for (int m = 0; m < R; ++m) zero_mode(z1, z2, m);
       }
       return;
     }
@@ -657,10 +675,8 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     };
     load_st(0);
     bool out_nz = false;  // a non-zero new mode outside the band
-    // where the zeros outside the band have to be stored
-    void* zero_out = rmode == RM_RHS ? a.rhs_out
-                     : s == 4 ? (a.th_out != a.th_n ? a.th_out : nullptr)
-                              : (a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
+    void* z1 = zero_out();
+    void* z2 = zero_acc();
     const bool ring_row = !scal && kp.ring_on && (rt.pos_lo <= rt.pos_hi || rt.neg_lo <= rt.neg_hi);
     const T tdt = (T)dt, dt2 = tdt * (T)0.5, dt3 = tdt / (T)3, dt6 = tdt / (T)6;
 #pragma unroll
@@ -771,10 +787,7 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
           if (!inb) out_nz |= !(o1.x == (T)0 && o1.y == (T)0 && o2.x == (T)0 && o2.y == (T)0);
         }
       }
-      if (!act && zero_out && valid) {
-        *rp.at(zero_out, m) = mkc<C>(0, 0);
-        if (pair) *rp.mir(zero_out, m) = mkc<C>(0, 0);
-      }
+      if (!act && valid) zero_mode(z1, z2, m);
       t1[m] = o1;
       t2[m] = o2;
       if (m + DEPTH < R && (tail || in_band(m + DEPTH))) issue(m + DEPTH);

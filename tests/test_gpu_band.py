@@ -109,3 +109,39 @@ def test_real_fields_at_any_element(P, N, prec):
     fh = pl.to_spectral(f)
     assert torch.equal(pl.to_spectral(odd), fh)
     assert torch.equal(pl.to_physical(fh, out=odd), pl.to_physical(fh))
+
+
+def stage_setup(P, N, prec, scheme, nu):
+    """A plan whose workspace holds another field's values at every mode, a
+    band-limited state and the oracle."""
+    g, go = P.make_grid(N, TWO_PI), O.make_grid(N, TWO_PI)
+    s = P.gSQGSolver(g, 1.0, nu, 4, precision=prec, scheme=scheme)
+    so = O.gSQGSolver(go, 1.0, nu, 4, scheme=scheme)
+    pl = s.plan()
+    dt = torch.complex128 if prec == "float64" else torch.complex64
+    other = torch.as_tensor(spectrum(N, "full", 8)).to("cuda", dt)
+    pl.step(other, torch.empty_like(other), 1e-3)
+    th = spectrum(N, "band", 9)
+    return pl, so, go, th, torch.as_tensor(th).to("cuda", dt)
+
+
+@pytest.mark.parametrize("N,prec", [(512, "float64"), (1024, "float32")])
+@pytest.mark.parametrize("scheme", ["ifrk4", "explicit"])
+@pytest.mark.parametrize("given", ["-f-f", "--f-", "---f", "p-f-", "pfpp"])
+def test_terms_at_some_stages_only(P, N, prec, scheme, given):
+    """Stage by stage: a spectral term (f), a physical one (p) or none (-)."""
+    dt = 1e-3
+    pl, so, go, th, t0 = stage_setup(P, N, prec, scheme, 0.3 / (N / 3.0) ** 4 / dt)
+    src = np.random.default_rng(3).standard_normal((N, N))
+    terms = {"f": 100.0 * spectrum(N, "full", 7), "p": go.dealias_mask * np.fft.fft2(src), "-": np.zeros((N, N))}
+    fd, pd = torch.as_tensor(terms["f"]).to(t0), torch.as_tensor(src).to("cuda", pl.rdtype)
+    out = torch.empty_like(t0)
+    pl.stage_begin(t0)
+    for s, k in enumerate(given, 1):
+        if k == "p":
+            pl.stage_physical(s, t0, out, dt, pd)
+        else:
+            pl.stage(s, t0, out, dt, fd if k == "f" else None)
+    order = iter(given)
+    ref = so.step({"theta_hat": th, "time": 0.0, "step": 0}, dt, forcing=lambda x: terms[next(order)])["theta_hat"]
+    assert rel(out, ref) < TOL[prec]
