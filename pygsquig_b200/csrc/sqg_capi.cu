@@ -437,10 +437,11 @@ int check_ready(const sqg_plan* pl) {
   return SQG_OK;
 }
 
-// One RK4 stage: column pass (with ring reduction) then row pass.
+// One RK4 stage: column pass (with ring reduction) then row pass.  separate:
+// the stages are separate calls, each with or without a term of the caller's.
 int run_stage(sqg_plan* pl, int s, const void* th_n, void* th_out, double dt, const void* extra,
               const double* phases, int stage_write, int do_p1, cudaStream_t st, RingCtl* ctl = nullptr,
-              const void* src_phys = nullptr, bool stage_read = false) {
+              const void* src_phys = nullptr, bool separate = false) {
   KP kp = make_kp(pl, dt);
   ColArgs ca = base_col(pl);
   ca.in_real = src_phys;
@@ -456,7 +457,7 @@ int run_stage(sqg_plan* pl, int s, const void* th_n, void* th_out, double dt, co
   ra.th_out = th_out;
   ra.extra = extra;
   ra.stage_write = stage_write;
-  ra.st_zero = stage_read ? 1 : 0;
+  ra.st_zero = separate ? 2 : (stage_write == SW_FULL ? 1 : 0);
   ra.do_p1 = do_p1;
   SQG_CUDA(launch_row(pl, kp, ra, st));
   return SQG_OK;

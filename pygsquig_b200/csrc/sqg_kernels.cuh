@@ -131,8 +131,8 @@ struct RowArgs {
   void* src_out[4];
   double gx[4], gy[4];
   int rpc;                        // row pairs per CTA (0: the compiled maximum RPC)
-  int st_zero;                    // 1: st_out is read outside the passes, and a later stage may add a term outside
-                                  // the band (stage 1 stores zeros there, in st_out and acc)
+  int st_zero;                    // zeros that stage 1 stores outside the band: 1 in st_out, which the caller may
+                                  // read; 2 also in acc, to which a later stage may add a term there
   unsigned char* tl;              // out-of-band flags of the field's row pairs (null: every row takes every mode)
   const unsigned char* tl_src;    // flags of src_h's rows (the theta its velocity came from)
 };
@@ -547,17 +547,16 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
         tile_tail |= t;
       }
     }
-    // Where the zeros outside the band have to be stored.  Stage buffer and
-    // accumulator: once a step, by stage 1 (no later stage touches them unless
-    // the row is flagged by then, and then it writes every mode), when
-    // the stages are separate calls: the caller reads the buffer, and a term
-    // given to a later stage meets the accumulator outside the band.
+    // Where the zeros outside the band have to be stored: the stage buffer and
+    // (when the stages are separate calls) the accumulator once a step, by stage
+    // 1.  No later stage touches them unless the row is flagged by then, and
+    // then it writes every mode.
     auto zero_out = [&]() -> void* {
       return rmode == RM_RHS ? a.rhs_out
              : stage == 4    ? (a.th_out != a.th_n ? a.th_out : nullptr)
                              : (stage == 1 && a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
     };
-    auto zero_acc = [&]() -> void* { return rmode == RM_STAGE && stage == 1 && a.st_zero ? a.acc : nullptr; };
+    auto zero_acc = [&]() -> void* { return rmode == RM_STAGE && stage == 1 && a.st_zero > 1 ? a.acc : nullptr; };
     auto zero_mode = [&](void* z1, void* z2, int m) {
       if (z1) {
         *rp.at(z1, m) = mkc<C>(0, 0);

@@ -145,3 +145,22 @@ def test_terms_at_some_stages_only(P, N, prec, scheme, given):
     order = iter(given)
     ref = so.step({"theta_hat": th, "time": 0.0, "step": 0}, dt, forcing=lambda x: terms[next(order)])["theta_hat"]
     assert rel(out, ref) < TOL[prec]
+
+
+@pytest.mark.parametrize("N,prec", [(512, "float64"), (1024, "float32")])
+def test_stage_buffer_of_a_whole_step(P, N, prec):
+    """The buffer holds the last stage's input at every mode after a step whose
+    stages store it (explicit scheme with a linear term)."""
+    from pygsquig_b200 import _lib
+
+    dt = 1e-3
+    pl, so, go, th, t0 = stage_setup(P, N, prec, "explicit", 0.3 / (N / 3.0) ** 4 / dt)
+    pl.step(t0, torch.empty_like(t0), dt)
+    x = th
+    for f in (0.5, 0.5, 1.0):
+        x = th + f * dt * so.compute_rhs(x)
+    buf = pl.buffer(_lib.SQG_BUF_STAGE, t0.dtype, t0.shape)
+    assert rel(buf, x) < TOL[prec]
+    k = np.abs(np.fft.fftfreq(N, 1.0 / N))
+    outside = torch.as_tensor(k[:, None] ** 2 + k[None, :] ** 2 > (N / 3.0 + 1) ** 2, device="cuda")
+    assert torch.count_nonzero(buf[outside]) == 0
