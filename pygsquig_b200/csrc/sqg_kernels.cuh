@@ -525,7 +525,9 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
         if (valid && j == 0) a.tl[p] = any ? 1 : 0;
         if (!any) return;
       } else {
-        const bool w = __any_sync(__activemask(), out);
+        // (every lane of the warp takes part, whatever has converged by here)
+        const unsigned lanes = (threadIdx.x | 31) < blockDim.x ? 0xffffffffu : (1u << (blockDim.x & 31)) - 1u;
+        const bool w = __any_sync(lanes, out);
         if ((threadIdx.x & 31) == 0) warp_out[threadIdx.x >> 5] = w;
       }
     }

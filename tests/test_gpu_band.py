@@ -164,3 +164,25 @@ def test_stage_buffer_of_a_whole_step(P, N, prec):
     k = np.abs(np.fft.fftfreq(N, 1.0 / N))
     outside = torch.as_tensor(k[:, None] ** 2 + k[None, :] ** 2 > (N / 3.0 + 1) ** 2, device="cuda")
     assert torch.count_nonzero(buf[outside]) == 0
+
+
+@pytest.mark.parametrize("N,prec", [(512, "float64"), (1024, "float32")])
+@pytest.mark.parametrize("p", [0, 3, 170, 171, -1])
+def test_one_mode_outside_at_every_element(P, N, prec, p):
+    """A row's flag sees one non-zero mode outside the band at whichever element it
+    stands (a single wave advects nothing: it stays as it is)."""
+    p = p % (N // 2 + 1)
+    s = P.gSQGSolver(P.make_grid(N, TWO_PI), 1.0, 0.0, 4, precision=prec, scheme="ifrk4")
+    pl = s.plan()
+    th = torch.zeros(N, N, dtype=pl.cdtype, device="cuda")
+    out = torch.empty_like(th)
+    worst = torch.zeros((), device="cuda", dtype=pl.rdtype)
+    for iy in range(N):
+        ky = min(iy, N - iy)
+        if p * p + ky * ky <= (N / 3.0 + 1) ** 2 or (p % (N // 2) == 0 and ky % (N // 2) == 0):
+            continue
+        th.zero_()
+        th[p, iy], th[-p % N, -iy % N] = 1 + 2j, 1 - 2j
+        pl.step(th, out, 1e-3)
+        worst = torch.maximum(worst, (out - th).abs().max())
+    assert float(worst) < 5 * TOL[prec]
