@@ -888,8 +888,9 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   };
   if constexpr (nfx_park(NFX)) fields(ha_smem);
   else fields(ha_reg);
+  if constexpr (N <= R) __syncthreads();  // warp_out; longer transforms hold barriers
   if (rmode == RM_P1 && a.tl && !tile_out && valid && j == 0) {
-    bool any = false;  // (the transforms' barriers lie between)
+    bool any = false;
     for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) any |= warp_out[w];
     a.tl[p] = any ? 1 : 0;
   }

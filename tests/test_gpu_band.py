@@ -186,3 +186,32 @@ def test_one_mode_outside_at_every_element(P, N, prec, p):
         pl.step(th, out, 1e-3)
         worst = torch.maximum(worst, (out - th).abs().max())
     assert float(worst) < 5 * TOL[prec]
+
+
+@pytest.mark.parametrize("prec", ["float64", "float32"])
+def test_smallest_ensemble_with_modes_outside(P, prec):
+    """N = 8: one transform pass, several warps to a block.  Members that hold one
+    mode outside the band each, against the single field's passes (every mode)."""
+    from pygsquig_b200.ensemble import EnsembleSolver, Member
+
+    N, modes = 8, [(p, iy) for p in range(5) for iy in range(8) if p * p + min(iy, 8 - iy) ** 2 >= 8]
+    z = np.zeros((N, N))
+    e = EnsembleSolver([Member(N, 1.0, z, [z], [1e-3]) for _ in modes], nu_p=1e-6, p=8, precision=prec)
+    band = spectrum(N, "band", 4)
+    solver = P.gSQGSolver(P.make_grid(N, TWO_PI), 1.0, 1e-6, 8, precision=prec, scheme="ifrk4")
+    ref = []
+    for i, (p, iy) in enumerate(modes):
+        th = band.copy()
+        th[p, iy], th[-p % N, -iy % N] = 0.3 + 0.2j, 0.3 - 0.2j
+        e.theta[i].copy_(torch.as_tensor(th))
+        e.scalars[i][0].copy_(torch.as_tensor(th))
+        st = {"theta_hat": e.theta[i].clone(), "time": 0.0, "step": 0}
+        ref.append(solver.multistep(st, 2, 1e-3)["theta_hat"])
+    e.multistep(2, 1e-3)
+    for a, b in zip(e.theta, ref):
+        assert rel(a, b.cpu().numpy()) < TOL[prec]
+    for i, (p, iy) in enumerate(modes):  # a scalar's mode outside decays by diffusion alone
+        if p % 4 == 0 and iy % 4 == 0:
+            continue  # its own conjugate
+        k2 = p * p + min(iy, N - iy) ** 2
+        assert abs(complex(e.scalars[i][0][p, iy].item()) / (0.3 + 0.2j) - np.exp(-2e-6 * k2)) < TOL[prec]
