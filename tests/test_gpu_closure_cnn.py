@@ -57,3 +57,39 @@ def test_cnn_training_reduces_loss():
         l1 = float(net.train_step(x, t))
     assert net.errors() == 0
     assert l1 < 0.3 * l0, (l0, l1)
+
+
+@pytest.mark.parametrize("off", [2, 4, 6])
+def test_gradients_of_tensors_at_any_channel_pair(off):
+    """Tensors of the first and last layers' gradients that start past a 16-byte
+    boundary give the bits of aligned ones."""
+    from pygsquig_b200 import _lib
+    from pygsquig_b200.build import build
+
+    build()
+    L, B, H, W = _lib.load(), 2, 3, 64
+    gen = torch.Generator(device="cuda").manual_seed(2)
+
+    def bf(*shape):
+        t = torch.randn(*shape, generator=gen, device="cuda").to(torch.bfloat16)
+        s = torch.zeros(t.numel() + 8, dtype=torch.bfloat16, device="cuda")[off : off + t.numel()].view(shape)
+        assert t.data_ptr() % 16 == 0 and s.data_ptr() % 16 == 2 * off
+        s.copy_(t)
+        return t, s
+
+    pad, z = bf(B, H + 2, W + 2, 64), bf(B, H, W, 64)
+    gy, x = torch.randn(B, H, W, generator=gen, device="cuda"), torch.randn(B, H, W, generator=gen, device="cuda")
+    w6 = torch.randn(9, 64, generator=gen, device="cuda")
+    red = torch.empty(296 * 640, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    got = []
+    for i in range(2):
+        outs = [torch.empty(640, device="cuda") for _ in range(3)]
+        for mode, a, gz in ((0, pad[i].data_ptr(), None), (1, None, pad[i].data_ptr()), (2, None, pad[i].data_ptr())):
+            assert L.closure_small_grad(mode, B, H, W, gy.data_ptr(), a, x.data_ptr(), gz, red.data_ptr(),
+                                        outs[mode].data_ptr(), st) == 0
+        g = bf(B, H + 2, W + 2, 64)[i]
+        assert L.closure_conv_out_dgrad(B, H, W, gy.data_ptr(), w6.data_ptr(), z[i].data_ptr(), g.data_ptr(), st) == 0
+        got.append(outs + [g.contiguous()])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
