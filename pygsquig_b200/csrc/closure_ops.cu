@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_small_grad_partial(int B, int H
                                                                     float* __restrict__ part) {
   constexpr int NT = MODE == 2 ? 0 : 9;  // taps
   __shared__ float stg[kWarps][3][34];
-  __shared__ float acc[kWarps][kRedStride];
+  __shared__ __align__(16) float acc[kWarps][kRedStride];  // (written in pairs)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane >> 3, g = lane & 7;
   float2 a[NT > 0 ? NT : 1][4], s[4];
