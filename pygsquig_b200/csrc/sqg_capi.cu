@@ -733,10 +733,12 @@ int sqg_plan_autotune(sqg_plan* pl, int32_t reps, void* stream) {
   int mr = 0, mn = 0;
   if (pl->d.precision == SQG_F64) shape_max_p<double>(pl->log2N, &mr, &mn);
   else shape_max_p<float>(pl->log2N, &mr, &mn);
-  void* th = pl->ws + pl->off_state;  // scratch input (zeroed) and output inside the workspace
+  void* th = pl->ws + pl->off_state;  // scratch input and output inside the workspace
   void* out = pl->ws + pl->off_stage;
   const size_t full = (size_t)pl->N * pl->N * pl->csize;
-  SQG_CUDA(cudaMemsetAsync(th, 0, full, st));
+  // no byte of it zero: values about 1e-38 (1e-303 in double), so that every row
+  // takes every mode, as a field fresh from physical space does
+  SQG_CUDA(cudaMemsetAsync(th, 1, full, st));
   const bool timing = pl->timing;
   pl->timing = false;
   const int r0 = pl->rpc, n0 = pl->np;

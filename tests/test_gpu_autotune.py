@@ -43,3 +43,17 @@ def test_every_shape_gives_identical_steps(N, prec):
     pl.autotune()
     with pytest.raises(ValueError):
         pl.set_shape(3, 0)
+
+
+@pytest.mark.parametrize("N,prec", [(512, "float64"), (1024, "float32"), (4096, "float32")])
+def test_shapes_are_timed_on_every_mode(N, prec):
+    """The tuner's right-hand sides (left in the stage buffer) are of a field with
+    modes everywhere, so no row of its passes is skipped."""
+    from pygsquig_b200 import _lib, gSQGSolver, make_grid
+    from pygsquig_b200.build import build
+
+    build()
+    pl = gSQGSolver(make_grid(N, 2 * math.pi), 1.0, 1.0, 2, precision=prec).plan()
+    pl.autotune(1)
+    rhs = pl.buffer(_lib.SQG_BUF_STAGE, pl.cdtype, (N, N)).flatten()
+    assert torch.count_nonzero(rhs[1:]) == N * N - 1
