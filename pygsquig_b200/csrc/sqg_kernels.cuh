@@ -61,8 +61,9 @@ enum FieldMode { FM_THETA = 0, FM_VEL = 1, FM_PHYS1 = 2, FM_SCAL = 3 };
 enum RowMode { RM_P1 = 0, RM_STAGE = 1, RM_RHS = 2, RM_SPEC = 3 };
 // Row-pass instances: one that reads its modes from the arguments (the batch
 // passes), and instances compiled for their modes alone: the stage passes of
-// theta and of the scalars (any stage, or one stage s = 1..4, RI_THETA_S1 + s -
-// 1, RI_SCAL_S1 + s - 1); the input passes (RM_P1) of theta, of the scalars, of
+// theta and of the scalars (any stage -- a single field's last one, without
+// transforms, and the multi-size passes -- or one stage s, RI_THETA_S1 + s - 1
+// with s = 1..4, RI_SCAL_S1 + s - 1 with s = 1..3); the input passes (RM_P1) of theta, of the scalars, of
 // the velocity and of a plain field; the right-hand side; the forward
 // transform.
 enum RowInst {

@@ -211,37 +211,43 @@ constexpr int row_inst(int rmode, int fmode) {
 }
 template <typename T, int L, int RI>
 cudaError_t launch_row_i(const KP& kp, const RowArgs& a, cudaStream_t st) {
-  constexpr int N = 1 << L, RPC = rows_per_cta<T, L>();
+  constexpr int N = 1 << L;
   if constexpr (RI == RI_THETA_STAGE || RI == RI_SCAL_STAGE) {
-    if (!a.do_p1) {  // last stage: its own radix, the compiled launch shape
-      constexpr int RPCX = rowx_rpc<T, L>();
-      RowArgs ax = a;
-      ax.rpc = 0;
-      return launch_pdl(k_row<T, L, rowx_radix<T, L>(), RPCX, rowx_depth<T, L>(), 0, RI>,
-                        dim3((N / 2 + 1 + RPCX - 1) / RPCX), dim3(RPCX * rowx_group<T, L>()),
-                        rowx_smem<T, L>(rowx_depth<T, L>()), st, kp, ax);
-    }
-  }
-  const int rpc = a.rpc > 0 ? a.rpc : RPC;
-  const int grid = (N / 2 + 1 + rpc - 1) / rpc;
-  return launch_pdl(k_row<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>(), RI>, dim3(grid),
-                    dim3(rpc * row_group<T, L>()), row_smem<T, L>() / RPC * rpc, st, kp, a);
-}
-template <typename T, int L, int RI0>
-cudaError_t launch_row_stage_i(const KP& kp, const RowArgs& a, cudaStream_t st) {
-  switch (a.stage) {
-    case 1: return launch_row_i<T, L, RI0>(kp, a, st);
-    case 2: return launch_row_i<T, L, RI0 + 1>(kp, a, st);
-    case 3: return launch_row_i<T, L, RI0 + 2>(kp, a, st);
-    default: return launch_row_i<T, L, RI0 + 3>(kp, a, st);
+    // last stage (no transforms): its own radix, the compiled launch shape
+    constexpr int RPCX = rowx_rpc<T, L>();
+    RowArgs ax = a;
+    ax.rpc = 0;
+    return launch_pdl(k_row<T, L, rowx_radix<T, L>(), RPCX, rowx_depth<T, L>(), 0, RI>,
+                      dim3((N / 2 + 1 + RPCX - 1) / RPCX), dim3(RPCX * rowx_group<T, L>()),
+                      rowx_smem<T, L>(rowx_depth<T, L>()), st, kp, ax);
+  } else {
+    constexpr int RPC = rows_per_cta<T, L>();
+    const int rpc = a.rpc > 0 ? a.rpc : RPC;
+    const int grid = (N / 2 + 1 + rpc - 1) / rpc;
+    return launch_pdl(k_row<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>(), RI>, dim3(grid),
+                      dim3(rpc * row_group<T, L>()), row_smem<T, L>() / RPC * rpc, st, kp, a);
   }
 }
 template <typename T, int L>
 cudaError_t launch_row_t(const KP& kp, const RowArgs& a, cudaStream_t st) {
   const int ri = row_inst(a.rmode, a.fmode);
-  if (a.do_p1 && a.stage >= 1 && a.stage <= 4) {
-    if (ri == RI_THETA_STAGE) return launch_row_stage_i<T, L, RI_THETA_S1>(kp, a, st);
-    if (ri == RI_SCAL_STAGE) return launch_row_stage_i<T, L, RI_SCAL_S1>(kp, a, st);
+  // stage passes with transforms: theta's stage 4 when the next step follows,
+  // a scalar's never
+  if (a.do_p1 && ri == RI_THETA_STAGE) {
+    switch (a.stage) {
+      case 1: return launch_row_i<T, L, RI_THETA_S1>(kp, a, st);
+      case 2: return launch_row_i<T, L, RI_THETA_S1 + 1>(kp, a, st);
+      case 3: return launch_row_i<T, L, RI_THETA_S1 + 2>(kp, a, st);
+      default: return launch_row_i<T, L, RI_THETA_S1 + 3>(kp, a, st);
+    }
+  }
+  if (a.do_p1 && ri == RI_SCAL_STAGE) {
+    switch (a.stage) {
+      case 1: return launch_row_i<T, L, RI_SCAL_S1>(kp, a, st);
+      case 2: return launch_row_i<T, L, RI_SCAL_S1 + 1>(kp, a, st);
+      case 3: return launch_row_i<T, L, RI_SCAL_S1 + 2>(kp, a, st);
+      default: return cudaErrorInvalidValue;
+    }
   }
   switch (ri) {
     case RI_THETA_STAGE: return launch_row_i<T, L, RI_THETA_STAGE>(kp, a, st);
@@ -298,22 +304,21 @@ cudaError_t shape_max_t(int* rpc, int* np) {
 }
 template <typename T, int L, int RI>
 cudaError_t set_row_attrs_i() {
-  constexpr int RPC = rows_per_cta<T, L>();
-  cudaError_t e = cudaFuncSetAttribute(k_row<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>(), RI>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T, L>());
-  if constexpr (RI == RI_THETA_STAGE || RI == RI_SCAL_STAGE) {  // the last-stage kernel: the stage instances
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_row<T, L, rowx_radix<T, L>(), rowx_rpc<T, L>(), rowx_depth<T, L>(), 0, RI>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowx_smem<T, L>(rowx_depth<T, L>()));
+  if constexpr (RI == RI_THETA_STAGE || RI == RI_SCAL_STAGE) {  // the last-stage kernel
+    return cudaFuncSetAttribute(k_row<T, L, rowx_radix<T, L>(), rowx_rpc<T, L>(), rowx_depth<T, L>(), 0, RI>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rowx_smem<T, L>(rowx_depth<T, L>()));
+  } else {
+    return cudaFuncSetAttribute(
+        k_row<T, L, row_radix<T, L>(), rows_per_cta<T, L>(), row_depth<T, L>(), row_nfx<T, L>(), RI>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T, L>());
   }
-  return e;
 }
-template <typename T, int L, int RI0>
-cudaError_t set_row_stage_attrs_i() {
-  cudaError_t e = set_row_attrs_i<T, L, RI0>();
-  if (e == cudaSuccess) e = set_row_attrs_i<T, L, RI0 + 1>();
-  if (e == cudaSuccess) e = set_row_attrs_i<T, L, RI0 + 2>();
-  if (e == cudaSuccess) e = set_row_attrs_i<T, L, RI0 + 3>();
+template <typename T, int L, int RI0, int RIN>
+cudaError_t set_row_attrs_to() {  // instances RI0 .. RIN - 1
+  const cudaError_t e = set_row_attrs_i<T, L, RI0>();
+  if constexpr (RI0 + 1 < RIN) {
+    if (e == cudaSuccess) return set_row_attrs_to<T, L, RI0 + 1, RIN>();
+  }
   return e;
 }
 template <typename T, int L, int CMX>
@@ -323,25 +328,8 @@ cudaError_t set_col_attrs_m() {
 }
 template <typename T, int L>
 cudaError_t set_attrs_t() {
-  cudaError_t e = set_row_attrs_i<T, L, RI_THETA_STAGE>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_SCAL_STAGE>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_THETA_P1>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_SCAL_P1>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_VEL_P1>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_PHYS_P1>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_RHS>();
-  if (e != cudaSuccess) return e;
-  e = set_row_attrs_i<T, L, RI_SPEC>();
-  if (e != cudaSuccess) return e;
-  e = set_row_stage_attrs_i<T, L, RI_THETA_S1>();
-  if (e != cudaSuccess) return e;
-  e = set_row_stage_attrs_i<T, L, RI_SCAL_S1>();
+  cudaError_t e = set_row_attrs_to<T, L, RI_THETA_STAGE, RI_SCAL_S1 + 3>();
+  if (e == cudaSuccess) e = set_row_attrs_to<T, L, RI_THETA_P1, RI_SPEC + 1>();
   if (e != cudaSuccess) return e;
   e = set_col_attrs_m<T, L, CM_THETA>();
   if (e == cudaSuccess) e = set_col_attrs_m<T, L, CM_SCAL>();
