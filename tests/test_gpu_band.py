@@ -215,3 +215,88 @@ def test_smallest_ensemble_with_modes_outside(P, prec):
             continue  # its own conjugate
         k2 = p * p + min(iy, N - iy) ** 2
         assert abs(complex(e.scalars[i][0][p, iy].item()) / (0.3 + 0.2j) - np.exp(-2e-6 * k2)) < TOL[prec]
+
+
+def rows_of(N, form, seed):
+    """As spectrum(); "mixed": of the rows beyond the band every fifth is held."""
+    if form != "mixed":
+        return spectrum(N, form, seed)
+    k = np.abs(np.fft.fftfreq(N, 1.0 / N))
+    keep = (k[:, None] <= N // 3) | (k[:, None] % 5 == 0)
+    return spectrum(N, "full", seed) * keep
+
+
+@pytest.fixture(scope="module")
+def threaded():
+    """The oracle's transforms on several threads (large grids)."""
+    O.set_fft_workers(16)
+    yield
+    O.set_fft_workers(1)
+
+
+@pytest.mark.parametrize("N", [2048, 4096])
+@pytest.mark.parametrize("form,other", [("rows", "mixed"), ("pair", "band"), ("mixed", "pair"), ("band", "full")])
+def test_large_step_with_some_rows_held(P, threaded, N, form, other):
+    """A step with a scalar whose rows differ from theta's: at these sizes the
+    rows beyond the band arrive in fetches of their own."""
+    dt = 1e-3
+    nu = 0.3 / (N / 3.0) ** 4 / dt
+    g, th, sa = P.make_grid(N, TWO_PI), rows_of(N, form, 1), rows_of(N, other, 3)
+    so = O.gSQGSolverWithScalars(O.make_grid(N, TWO_PI), 0.5, nu, 4, scheme="ifrk4", passive_scalars={
+        "a": {"kappa": 1e-3, "source": O.MeanGradientSource(1.0, 0.5)}})
+    ref = so.step({"theta_hat": th, "time": 0.0, "step": 0, "scalars": {"a": sa}}, dt)
+    for prec, cdt in (("float64", torch.complex128), ("float32", torch.complex64)):
+        s = P.gSQGSolverWithScalars(g, 0.5, nu, 4, precision=prec, scheme="ifrk4", passive_scalars={
+            "a": {"kappa": 1e-3, "source": P.MeanGradientSource(1.0, 0.5)}})
+        t, q = (torch.as_tensor(x).to("cuda", cdt) for x in (th, sa))
+        st = s.step({"theta_hat": t, "time": 0.0, "step": 0, "scalar_state": P.MultiScalarState({"a": q}, 0.0, {})}, dt)
+        assert rel(st["theta_hat"], ref["theta_hat"]) < TOL[prec]
+        assert rel(st["scalar_state"].scalars["a"], ref["scalars"]["a"]) < TOL[prec]
+        # from the second step on, the last stage sets the flags of the next
+        s1 = P.gSQGSolver(g, 0.5, nu, 4, precision=prec, scheme="ifrk4")
+        x = {"theta_hat": t, "time": 0.0, "step": 0}
+        two = s1.step(s1.step(x, dt), dt)["theta_hat"].cpu().numpy()
+        assert rel(s1.multistep(x, 2, dt)["theta_hat"], two) < TOL[prec]
+
+
+@pytest.mark.parametrize("form", ["rows", "pair", "mixed", "band"])
+@pytest.mark.parametrize("N", [2048, 4096])
+def test_large_rhs_and_velocity_with_some_rows_held(P, threaded, N, form):
+    th, go = rows_of(N, form, 1), O.make_grid(N, TWO_PI)
+    so = O.gSQGSolver(go, 0.5, 1e-8, 2)
+    rhs, vel = so.compute_rhs(th), so.compute_velocity(th)
+    for prec in ("float64", "float32"):
+        s = P.gSQGSolver(P.make_grid(N, TWO_PI), 0.5, 1e-8, 2, precision=prec)
+        t = torch.as_tensor(th).cuda()
+        assert rel(s.compute_rhs(t), rhs) < TOL[prec]
+        for a, b in zip(s.compute_velocity(t), vel):
+            assert rel(a, b) < TOL[prec]
+
+
+@pytest.mark.parametrize("sizes", [(32, 64), (128, 512), (256, 1024)])
+@pytest.mark.parametrize("prec", ["float64", "float32"])
+def test_ensemble_members_with_some_rows_held(P, sizes, prec):
+    """Theta and scalars hold different rows: the unified passes (128, 512) and
+    the passes class by class."""
+    from pygsquig_b200.ensemble import EnsembleSolver, Member
+
+    forms = [("band", "full"), ("full", "band"), ("pair", "rows"), ("mixed", "pair"), ("band", "band")]
+    members = [(N, f) for N in sizes for f in (forms if N < 1024 else forms[2:4])]
+    nu, dt = 0.3 / (max(sizes) / 3.0) ** 8 / 1e-3, 1e-3
+    e = EnsembleSolver([Member(N, 0.5, np.zeros((N, N)), [np.zeros((N, N))] * 2, [1e-3, 1e-4]) for N, _ in members],
+                       nu_p=nu, p=8, precision=prec)
+    refs = []
+    for i, (N, (a, b)) in enumerate(members):
+        th, s1, s2 = rows_of(N, a, i), rows_of(N, b, 40 + i), rows_of(N, a, 80 + i)
+        for t, x in zip([e.theta[i]] + e.scalars[i], (th, s1, s2)):
+            t.copy_(torch.as_tensor(x))
+        so = O.gSQGSolverWithScalars(O.make_grid(N, TWO_PI), 0.5, nu, 8, scheme="ifrk4", passive_scalars={
+            "a": {"kappa": 1e-3, "source": None}, "b": {"kappa": 1e-4, "source": None}})
+        st = {"theta_hat": th, "time": 0.0, "step": 0, "scalars": {"a": s1, "b": s2}}
+        for _ in range(2):
+            st = so.step(st, dt)
+        refs.append([st["theta_hat"], st["scalars"]["a"], st["scalars"]["b"]])
+    e.multistep(2, dt)
+    for i, ref in enumerate(refs):
+        for t, x in zip([e.theta[i]] + e.scalars[i], ref):
+            assert rel(t, x) < TOL[prec], (members[i], i)
