@@ -335,18 +335,13 @@ __device__ __forceinline__ int ring_ord(const RowTab& rt, int iy) {
   return -1;
 }
 
-// Scaled ring forcing of stage s at (row of rt, iy), zero off the ring; and as
-// a call (see linear_op_call).
+// Scaled ring forcing of stage s at (row of rt, iy), zero off the ring.
 template <typename C>
 __device__ __forceinline__ C ring_force(const KP& kp, const RowTab& rt, int iy, int s) {
   const int o = ring_ord(rt, iy);
   if (o < 0) return mkc<C>(0, 0);
   const double2 f = kp.ringF[(size_t)(s - 1) * kp.n_ring + o];
   return mkc<C>(f.x, f.y);
-}
-template <typename C>
-__device__ __noinline__ C ring_force_call(const KP& kp, const RowTab* rt, int iy, int s) {
-  return ring_force<C>(kp, *rt, iy, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -466,7 +461,9 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   // modes fixed by the instance (RI), else read from the arguments
   const int rmode = ri_rmode(RI) >= 0 ? ri_rmode(RI) : a.rmode;
   const int fmode = ri_fmode(RI) >= 0 ? ri_fmode(RI) : a.fmode;
-  const int stage = ri_stage(RI) > 0 ? ri_stage(RI) : a.stage;
+  // (without transforms: the last stage; as a value read at run time, its code
+  // held every stage's: N = 256 FP64 4.5 us a pass instead of 3.6)
+  const int stage = NFX == 0 ? 4 : (ri_stage(RI) > 0 ? ri_stage(RI) : a.stage);
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N;
   constexpr int G = N / R;
@@ -716,13 +713,8 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
         const int iy = j + m * G;
         const bool ring = ring_row && ((iy >= rt.pos_lo && iy <= rt.pos_hi) || (iy >= rt.neg_lo && iy <= rt.neg_hi));
         if (ring) {
-          if constexpr (CALLS) {
-            n1 = cadd(n1, ring_force_call<C>(kp, kp.rows + p, iy, s));
-            if (pair) n2 = cadd(n2, ring_force_call<C>(kp, kp.rows + pp, EL::mirror(j, m), s));
-          } else {
-            n1 = cadd(n1, ring_force<C>(kp, rt, iy, s));
-            if (pair) n2 = cadd(n2, ring_force<C>(kp, kp.rows[pp], EL::mirror(j, m), s));
-          }
+          n1 = cadd(n1, ring_force<C>(kp, rt, iy, s));
+          if (pair) n2 = cadd(n2, ring_force<C>(kp, kp.rows[pp], EL::mirror(j, m), s));
         }
         if (a.extra) {
           n1 = cadd(n1, *rp.at(a.extra, m));
