@@ -1060,18 +1060,24 @@ __device__ __forceinline__ void col_first_load(const typename Cplx<T>::type* z, 
 }
 
 // Where some row beyond pmax is live, all were fetched: the unflagged ones,
-// unwritten in xh, become zero in the raw slots z of a column pair (by the
-// pair's G threads; the caller's barriers lie around it).  Not in the radix-16
-// theta pass, which is at its register cap: the flags in its load's condition
-// measured 159 us against 174 at N = 4096 (scalars' pass the other way round,
-// 113 against 108; multi-size passes 80 against 67).
+// unwritten in xh, become zero in the raw slots of n buffers of a column pair,
+// z, z + sz, ... (by the pair's G threads; the caller's barriers lie around it).
+// The buffers share each flag's load, and the loads are independent.
+// Not in the radix-16 theta pass, which is at its register cap: the flags in its
+// load's condition measured 159 us against 174 at N = 4096 (scalars' pass the
+// other way round, 113 against 108; multi-size passes 80 against 67).
 template <typename C>
-__device__ __noinline__ void col_zero_rows(C* z, int j, int G, int pmax, int H, const unsigned char* tl) {
-  for (int kx = pmax + 1 + j; kx <= H; kx += G)
-    if (!tl[kx]) {
-      z[2 * kx].x = z[2 * kx].y = 0;
-      z[2 * kx + 1].x = z[2 * kx + 1].y = 0;
+__device__ __noinline__ void col_zero_rows(C* z, int sz, int n, int j, int G, int pmax, int H,
+                                           const unsigned char* __restrict__ tl) {
+#pragma unroll 4
+  for (int kx = pmax + 1 + j; kx <= H; kx += G) {
+    if (tl[kx]) continue;
+    for (int b = 0; b < n; ++b) {
+      C* q = z + b * sz + 2 * kx;
+      q[0].x = q[0].y = 0;
+      q[1].x = q[1].y = 0;
     }
+  }
 }
 
 template <typename T, int LOG2N>
@@ -1155,8 +1161,8 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
   constexpr bool BYROW = R == 16 && CMX == CM_THETA;
   const unsigned char *tl = nullptr, *tl2 = nullptr;  // flags, where a row beyond pmax is live
   bool dead = false;                                  // ... and another is not
-  auto zero_rows = [&](int b, const unsigned char* t) {
-    col_zero_rows(gbuf + b * SZ, j, G, pin, H, t);
+  auto zero_rows = [&](int step, int n, const unsigned char* t, int b = 0) {  // buffers b, b + step, ...
+    col_zero_rows(gbuf + b * SZ, step * SZ, n, j, G, pin, H, t);
   };
   auto first_load = [&](int b, C (&x)[R]) {
     col_first_load<T, LOG2N, R, BYROW>(gbuf + b * SZ, j, x, !BYROW && tl ? H : pin, tl);
@@ -1203,7 +1209,7 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     __syncthreads();
     tile_wait(0, 0);
     if (dead) {
-      for (int f = 0; f < nf; ++f) zero_rows(f, tl);
+      zero_rows(1, nf, tl);
       __syncthreads();
     }
     if constexpr (CMX != CM_VEL) {
@@ -1290,7 +1296,12 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     __syncthreads();
     tile_wait(0, 0);
     if (dead) {
-      for (int f = 0; f < 4; ++f) zero_rows(f, (f & 1) ? tl2 : tl);
+      if (tl2 == tl) {
+        zero_rows(1, 4, tl);
+      } else {
+        zero_rows(2, 2, tl);
+        zero_rows(2, 2, tl2, 1);
+      }
       __syncthreads();
     }
     C V[4][R];
@@ -1333,8 +1344,7 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
       tile_wait(0, (uint32_t)rd);
       if (NBUF == 3 && rd == 1) tile_wait(1, 0);
       if (dead) {
-        zero_rows(NBUF == 3 && rd == 1 ? 2 : 0, tl);
-        zero_rows(NBUF == 3 && rd == 1 ? 0 : 1, tl);
+        zero_rows(NBUF == 3 && rd == 1 ? 2 : 1, 2, tl);
         __syncthreads();
       }
       C V[2][R];
