@@ -1473,30 +1473,41 @@ struct sqg_batch {
 namespace {
 
 template <typename T>
-cudaError_t launch_row_batch_p(int log2n, const KP* kps, const RowArgs* as, int m, cudaStream_t st) {
-  SQG_DISPATCH(log2n, launch_row_batch_t, kps, as, m, st);
+cudaError_t launch_row_batch_p(int log2n, const KP* kps, const RowArgs* as, int m, int ri, cudaStream_t st) {
+  SQG_DISPATCH(log2n, launch_row_batch_t, kps, as, m, ri, st);
 }
 template <typename T>
-cudaError_t launch_col_batch_p(int log2n, const KP* kps, const ColArgs* as, int m, cudaStream_t st) {
-  SQG_DISPATCH(log2n, launch_col_batch_t, kps, as, m, st);
+cudaError_t launch_col_batch_p(int log2n, const KP* kps, const ColArgs* as, int m, int cm, cudaStream_t st) {
+  SQG_DISPATCH(log2n, launch_col_batch_t, kps, as, m, cm, st);
 }
 template <typename T>
 cudaError_t set_batch_attrs_p(int log2n) {
   SQG_DISPATCH(log2n, set_batch_attrs_t);
 }
 
-cudaError_t brow(sqg_batch* b, const KP* kps, const RowArgs* as, int m, cudaStream_t st) {
+// All members of a launch are of one kind: the row instance ri, the column mode cm.
+cudaError_t brow(sqg_batch* b, const KP* kps, const RowArgs* as, int m, int ri, cudaStream_t st) {
   if (m == 0) return cudaSuccess;
   b->launches++;
-  return b->d.precision == SQG_F64 ? launch_row_batch_p<double>(b->log2N, kps, as, m, st)
-                                   : launch_row_batch_p<float>(b->log2N, kps, as, m, st);
+  return b->d.precision == SQG_F64 ? launch_row_batch_p<double>(b->log2N, kps, as, m, ri, st)
+                                   : launch_row_batch_p<float>(b->log2N, kps, as, m, ri, st);
 }
-cudaError_t bcol(sqg_batch* b, const KP* kps, const ColArgs* as, int m, cudaStream_t st) {
+cudaError_t bcol(sqg_batch* b, const KP* kps, const ColArgs* as, int m, int cm, cudaStream_t st) {
   if (m == 0) return cudaSuccess;
   b->launches++;
-  return b->d.precision == SQG_F64 ? launch_col_batch_p<double>(b->log2N, kps, as, m, st)
-                                   : launch_col_batch_p<float>(b->log2N, kps, as, m, st);
+  return b->d.precision == SQG_F64 ? launch_col_batch_p<double>(b->log2N, kps, as, m, cm, st)
+                                   : launch_col_batch_p<float>(b->log2N, kps, as, m, cm, st);
 }
+
+// Whether theta's (the scalars') passes of an ensemble's size class keep flags of
+// their rows.  They pay where rows are skipped and cost where none is, the less
+// the longer a row; a theta's rows outside the band are soon emptied by
+// hyperviscosity, a scalar's diffusion leaves round-off there for thousands of
+// steps.  Three steps, every row live (after the second slash: none outside the band),
+// with both flags and without: N = 64 x 48 FP32 320 and 293 us / 283 and 290;
+// 128 x 48 FP64 1251 and 1181 / 921 and 1199; 256 x 24 FP64 2458 and 2313 / 1867
+// and 2309; 512 x 12 FP32 1994 and 2162 / 1639 and 2153.
+bool batch_flags(int N, bool theta) { return N >= (theta ? 128 : 256); }
 
 // Builds and uploads every member's pass arguments for time step dt.
 int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
@@ -1527,7 +1538,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     a.th_n = b->mem[i].theta;
     a.th_out = b->mem[i].theta;
     a.do_p1 = 1;
-    a.tl = mb + b->m_tl;
+    a.tl = batch_flags(b->N, true) ? mb + b->m_tl : nullptr;
     p1[i] = a;
     p1[i].rmode = RM_P1;
     for (int s = 1; s <= 4; ++s) {
@@ -1568,7 +1579,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     a.th_out = b->mem[i].scalars[q];
     a.kappa = b->mem[i].kappa[q];
     a.do_p1 = 1;
-    a.tl = sb + b->s_tl;
+    a.tl = batch_flags(b->N, false) ? sb + b->s_tl : nullptr;
     sp1[k] = a;
     sp1[k].rmode = RM_P1;
     const bool sexp = b->d.scheme == SQG_EXPLICIT_RK4 && a.kappa != 0.0;
@@ -1595,7 +1606,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     cv.cmode = CM_SCALV;
     cv.xh = mb + b->m_xh;
     cv.xh2 = a.xh;
-    cv.tl = mb + b->m_tl;
+    cv.tl = batch_flags(b->N, true) ? mb + b->m_tl : nullptr;
     cv.tl2 = a.tl;
     cv.out0 = q == 0 ? mb + b->m_uv : nullptr;
     scolv[k] = cv;
@@ -1627,16 +1638,16 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
 int batch_step_launches(sqg_batch* b, cudaStream_t st) {
   const int M = b->M, S = b->S;
   for (int s = 1; s <= 4; ++s) {
-    SQG_CUDA(bcol(b, b->d_kp, b->d_col, M, st));
-    SQG_CUDA(brow(b, b->d_kp, b->d_row + (size_t)(s - 1) * M, M, st));
+    SQG_CUDA(bcol(b, b->d_kp, b->d_col, M, CM_THETA, st));
+    SQG_CUDA(brow(b, b->d_kp, b->d_row + (size_t)(s - 1) * M, M, RI_THETA_STAGE, st));
   }
   if (S > 0) {
     // u + i v of theta_{n+1} from the stage-4 transforms, then the scalars
-    SQG_CUDA(bcol(b, b->d_kp, b->d_vel, M, st));
-    SQG_CUDA(brow(b, b->d_kps, b->d_sp1, S, st));
+    SQG_CUDA(bcol(b, b->d_kp, b->d_vel, M, CM_VEL, st));
+    SQG_CUDA(brow(b, b->d_kps, b->d_sp1, S, RI_SCAL_P1, st));
     for (int s = 1; s <= 4; ++s) {
-      SQG_CUDA(bcol(b, b->d_kps, b->d_scol, S, st));
-      SQG_CUDA(brow(b, b->d_kps, b->d_srow + (size_t)(s - 1) * S, S, st));
+      SQG_CUDA(bcol(b, b->d_kps, b->d_scol, S, CM_SCAL, st));
+      SQG_CUDA(brow(b, b->d_kps, b->d_srow + (size_t)(s - 1) * S, S, RI_SCAL_STAGE, st));
     }
   }
   return SQG_OK;
@@ -1754,7 +1765,7 @@ int sqg_batch_multistep(sqg_batch* b, int32_t n_steps, double dt, int32_t use_gr
   }
   b->launches = 0;
   // theta P1 of every member's input state
-  SQG_CUDA(brow(b, b->d_kp, b->d_p1, b->M, st));
+  SQG_CUDA(brow(b, b->d_kp, b->d_p1, b->M, RI_THETA_P1, st));
   if (!use_graph) {
     for (int n = 0; n < n_steps; ++n)
       if ((rc = batch_step_launches(b, st)) != SQG_OK) return rc;

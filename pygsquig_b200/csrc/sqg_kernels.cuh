@@ -59,27 +59,23 @@ struct RowTab {
 // written nor read nor transformed beyond pmax, where the mask discards it.
 enum FieldMode { FM_THETA = 0, FM_VEL = 1, FM_PHYS1 = 2, FM_SCAL = 3 };
 enum RowMode { RM_P1 = 0, RM_STAGE = 1, RM_RHS = 2, RM_SPEC = 3 };
-// Row-pass instances: one that reads its modes from the arguments (the batch
-// passes), and instances compiled for their modes alone: the stage passes of
+// Row-pass instances, each compiled for its modes alone: the stage passes of
 // theta and of the scalars (any stage -- a single field's last one, without
-// transforms, and the multi-size passes -- or one stage s, RI_THETA_S1 + s - 1
-// with s = 1..4, RI_SCAL_S1 + s - 1 with s = 1..3); the input passes (RM_P1) of theta, of the scalars, of
+// transforms, and the passes of many fields -- or one stage s, RI_THETA_S1 + s -
+// 1 with s = 1..4, RI_SCAL_S1 + s - 1 with s = 1..3); the input passes (RM_P1) of theta, of the scalars, of
 // the velocity and of a plain field; the right-hand side; the forward
 // transform.
 enum RowInst {
-  RI_ANY = 0, RI_THETA_STAGE = 1, RI_SCAL_STAGE = 2, RI_THETA_S1 = 3, RI_SCAL_S1 = 7,
+  RI_THETA_STAGE = 1, RI_SCAL_STAGE = 2, RI_THETA_S1 = 3, RI_SCAL_S1 = 7,
   RI_THETA_P1 = 11, RI_SCAL_P1 = 12, RI_VEL_P1 = 13, RI_PHYS_P1 = 14, RI_RHS = 15, RI_SPEC = 16
 };
 __host__ __device__ constexpr int ri_fmode(int ri) {
   return (ri == RI_THETA_STAGE || ri == RI_THETA_P1 || ri == RI_RHS || ri == RI_SPEC ||
           (ri >= RI_THETA_S1 && ri < RI_SCAL_S1)) ? FM_THETA
-         : ((ri == RI_SCAL_STAGE || ri == RI_SCAL_P1 || (ri >= RI_SCAL_S1 && ri < RI_SCAL_S1 + 4))
-                ? FM_SCAL
-                : (ri == RI_VEL_P1 ? FM_VEL : (ri == RI_PHYS_P1 ? FM_PHYS1 : -1)));
+         : (ri == RI_VEL_P1 ? FM_VEL : (ri == RI_PHYS_P1 ? FM_PHYS1 : FM_SCAL));
 }
 __host__ __device__ constexpr int ri_rmode(int ri) {
-  return ri == RI_ANY ? -1
-         : ri == RI_RHS ? RM_RHS
+  return ri == RI_RHS ? RM_RHS
          : ri == RI_SPEC ? RM_SPEC : (ri >= RI_THETA_P1 ? RM_P1 : RM_STAGE);
 }
 __host__ __device__ constexpr int ri_stage(int ri) {
@@ -456,14 +452,22 @@ __device__ __forceinline__ void row_fields(const KP& kp, const RowArgs& a, HA ha
 // cp.async ahead of use; the first DEPTH chunks are requested before the
 // forward FFT of the J row, so their latency hides behind it.
 // BATCH: a pass of many fields, its arguments read from device arrays.
-template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI = RI_ANY, bool BATCH = RI == RI_ANY>
+template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI, bool BATCH = false>
 __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int tile) {
-  // modes fixed by the instance (RI), else read from the arguments
-  const int rmode = ri_rmode(RI) >= 0 ? ri_rmode(RI) : a.rmode;
-  const int fmode = ri_fmode(RI) >= 0 ? ri_fmode(RI) : a.fmode;
+  constexpr int rmode = ri_rmode(RI), fmode = ri_fmode(RI);
   // (without transforms: the last stage; as a value read at run time, its code
   // held every stage's: N = 256 FP64 4.5 us a pass instead of 3.6)
   const int stage = NFX == 0 ? 4 : (ri_stage(RI) > 0 ? ri_stage(RI) : a.stage);
+  // (read once: batches keep their arguments in memory that the pass's stores
+  // might alias, and a reload after every store made the scalars' last pass of
+  // N = 128 FP64 ensembles 8.0 us instead of 5.6; batches carry no extra terms or
+  // sources)
+  const void *const th_n = a.th_n, *const jh = a.jh;
+  const void *const extra = BATCH ? nullptr : a.extra, *const src_h = BATCH ? nullptr : a.src_h;
+  void *const th_out = a.th_out, *const acc = a.acc, *const st_out = a.st_out, *const rhs_out = a.rhs_out;
+  unsigned char* const tl = a.tl;
+  const unsigned char* const tl_src = BATCH ? nullptr : a.tl_src;
+  const int stage_write = a.stage_write, st_zero = BATCH ? 0 : a.st_zero, do_p1 = a.do_p1;
   using C = typename Cplx<T>::type;
   constexpr int N = 1 << LOG2N;
   constexpr int G = N / R;
@@ -508,10 +512,10 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   if (rmode == RM_P1) {
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      t1[m] = *rp.at(a.th_n, m);
-      t2[m] = *rp.mir(a.th_n, m);
+      t1[m] = *rp.at(th_n, m);
+      t2[m] = *rp.mir(th_n, m);
     }
-    if (a.tl) {
+    if (tl) {
       bool out = false;
 #pragma unroll
       for (int m = 0; m < R; ++m)
@@ -520,7 +524,7 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
       // leave, else collected by warp and stored after the transforms
       if (tile_out) {
         const int any = __syncthreads_or(out);
-        if (valid && j == 0) a.tl[p] = any ? 1 : 0;
+        if (valid && j == 0) tl[p] = any ? 1 : 0;
         if (!any) return;
       } else {
         // (every lane of the warp takes part, whatever has converged by here)
@@ -532,14 +536,14 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   } else {
     // Whether this row (and any row of the block, block-uniform) has modes
     // outside the band, or its source does.
-    bool tail = a.tl == nullptr || a.extra != nullptr, src_row = true;
+    bool tail = tl == nullptr || extra != nullptr, src_row = true;
     bool tile_tail = tail;
-    if (a.tl && rmode != RM_SPEC) {
+    if (tl && rmode != RM_SPEC) {
       for (int g = 0; g < rpc; ++g) {
         const int pg = tile * rpc + g <= H ? tile * rpc + g : H;
-        bool t = a.tl[pg] != 0;
-        if (a.tl_src) {
-          const bool ts = a.tl_src[pg] != 0;
+        bool t = tl[pg] != 0;
+        if (tl_src) {
+          const bool ts = tl_src[pg] != 0;
           if (pg == p) src_row = ts || p <= kp.pmax;  // unwritten source rows are zero
           t |= ts;
         }
@@ -552,11 +556,11 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     // 1.  No later stage touches them unless the row is flagged by then, and
     // then it writes every mode.
     auto zero_out = [&]() -> void* {
-      return rmode == RM_RHS ? a.rhs_out
-             : stage == 4    ? (a.th_out != a.th_n ? a.th_out : nullptr)
-                             : (stage == 1 && a.stage_write == SW_FULL && a.st_zero ? a.st_out : nullptr);
+      return rmode == RM_RHS ? rhs_out
+             : stage == 4    ? (th_out != th_n ? th_out : nullptr)
+                             : (stage == 1 && stage_write == SW_FULL && st_zero ? st_out : nullptr);
     };
-    auto zero_acc = [&]() -> void* { return rmode == RM_STAGE && stage == 1 && a.st_zero > 1 ? a.acc : nullptr; };
+    auto zero_acc = [&]() -> void* { return rmode == RM_STAGE && stage == 1 && st_zero > 1 ? acc : nullptr; };
     auto zero_mode = [&](void* z1, void* z2, int m) {
       if (z1) {
         *rp.at(z1, m) = mkc<C>(0, 0);
@@ -585,12 +589,12 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     auto issue = [&](int m) {
       C* slot = pf + (size_t)(m % DEPTH) * 4 * G + j;
       if (pf_th) {
-        cp_async_elem(slot, rp.at(a.th_n, m), (int)sizeof(C));
-        if (pair) cp_async_elem(slot + G, rp.mir(a.th_n, m), (int)sizeof(C));
+        cp_async_elem(slot, rp.at(th_n, m), (int)sizeof(C));
+        if (pair) cp_async_elem(slot + G, rp.mir(th_n, m), (int)sizeof(C));
       }
       if (pf_acc) {
-        cp_async_elem(slot + 2 * G, rp.at(a.acc, m), (int)sizeof(C));
-        if (pair) cp_async_elem(slot + 3 * G, rp.mir(a.acc, m), (int)sizeof(C));
+        cp_async_elem(slot + 2 * G, rp.at(acc, m), (int)sizeof(C));
+        if (pair) cp_async_elem(slot + 3 * G, rp.mir(acc, m), (int)sizeof(C));
       }
     };
 #pragma unroll
@@ -600,7 +604,7 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     // leaves the rows beyond the band unwritten: the mask discards them)
     const bool use_j = rmode == RM_SPEC || !tile_out;
 #pragma unroll
-    for (int m = 0; m < R; ++m) v[m] = use_j ? *rp.at(a.jh, m) : mkc<C>(0, 0);
+    for (int m = 0; m < R; ++m) v[m] = use_j ? *rp.at(jh, m) : mkc<C>(0, 0);
 #pragma unroll
     for (int m = 0; m < DEPTH; ++m)
       if (tail && !in_band(m)) issue(m);
@@ -615,7 +619,7 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     const bool use_exp = rmode == RM_STAGE && !explicit_lin && s < 4;
     const bool use_lin = rmode == RM_RHS || explicit_lin || s < 4;
     // (a scalar's operator is short: at its elements again, N = 256 FP32 step 42.5 -> 39 us)
-    constexpr bool CALLS = (LOG2N <= 9 && ri_fmode(RI) != FM_SCAL) || BATCH;
+    constexpr bool CALLS = LOG2N <= 9 && ri_fmode(RI) != FM_SCAL && !BATCH;
     auto linear = [&](int m, T& e, T& e2, T& lt) {
       e = e2 = (T)1;
       lt = (T)0;
@@ -650,19 +654,19 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
       if (valid) {
 #pragma unroll
         for (int m = 0; m < R; ++m) {
-          *rp.at(a.rhs_out, m) = v[m];
-          if (pair) *rp.mir(a.rhs_out, m) = cconj(v[m]);
+          *rp.at(rhs_out, m) = v[m];
+          if (pair) *rp.mir(rhs_out, m) = cconj(v[m]);
         }
       }
       return;
     }
-    const void* st_in = s == 1 ? a.th_n : a.st_in;
+    const void* st_in = s == 1 ? th_n : a.st_in;
     // the scalar's source term is read one chunk ahead, ahead of the wait
     // for the chunk's prefetched values, so that its latency overlaps the
     // element updates of the chunk before
-    const bool use_src = scal && a.src_h != nullptr && src_row;
+    const bool use_src = scal && src_h != nullptr && src_row;
     C sh_next = mkc<C>(0, 0);
-    if (use_src) sh_next = *rp.at(a.src_h, 0);
+    if (use_src) sh_next = *rp.at(src_h, 0);
     // the explicit scheme's stage input likewise
     const bool use_st = (explicit_lin && s > 1 && rmode == RM_STAGE) || rmode == RM_RHS;
     C x_next1 = mkc<C>(0, 0), x_next2 = mkc<C>(0, 0);
@@ -676,13 +680,13 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
     bool out_nz = false;  // a non-zero new mode outside the band
     void* z1 = zero_out();
     void* z2 = zero_acc();
-    const bool ring_row = !scal && kp.ring_on && (rt.pos_lo <= rt.pos_hi || rt.neg_lo <= rt.neg_hi);
+    const bool ring_row = !BATCH && !scal && kp.ring_on && (rt.pos_lo <= rt.pos_hi || rt.neg_lo <= rt.neg_hi);
     const T tdt = (T)dt, dt2 = tdt * (T)0.5, dt3 = tdt / (T)3, dt6 = tdt / (T)6;
 #pragma unroll
     for (int m = 0; m < R; ++m) {
       const int my = EL::mag(j, m);
       const C sh = sh_next;
-      if (use_src && m + 1 < R) sh_next = *rp.at(a.src_h, m + 1);
+      if (use_src && m + 1 < R) sh_next = *rp.at(src_h, m + 1);
       const C xi1 = x_next1, xi2 = x_next2;
       if (m + 1 < R) load_st(m + 1);
       // chunk m has landed (groups complete in order)
@@ -716,14 +720,14 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
           n1 = cadd(n1, ring_force<C>(kp, rt, iy, s));
           if (pair) n2 = cadd(n2, ring_force<C>(kp, kp.rows[pp], EL::mirror(j, m), s));
         }
-        if (a.extra) {
-          n1 = cadd(n1, *rp.at(a.extra, m));
-          if (pair) n2 = cadd(n2, *rp.mir(a.extra, m));
+        if (extra) {
+          n1 = cadd(n1, *rp.at(extra, m));
+          if (pair) n2 = cadd(n2, *rp.mir(extra, m));
         }
         if (rmode == RM_RHS) {
           if (wr) {
-            *rp.at(a.rhs_out, m) = cadd(n1, cscale(xi1, Lt));
-            if (pair) *rp.mir(a.rhs_out, m) = cadd(n2, cscale(xi2, Lt));
+            *rp.at(rhs_out, m) = cadd(n1, cscale(xi1, Lt));
+            if (pair) *rp.mir(rhs_out, m) = cadd(n2, cscale(xi2, Lt));
           }
         } else {
           C k1v = n1, k2v = n2;
@@ -739,24 +743,24 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
           if (s == 1) {
             // acc = E^2 (th + dt/6 k) ; th2 = E (th + dt/2 k)
             const C a1 = cscale(cadd(xs1, cscale(k1v, dt6)), E2);
-            if (wr) *rp.at(a.acc, m) = a1;
+            if (wr) *rp.at(acc, m) = a1;
             o1 = cscale(cadd(xs1, cscale(k1v, dt2)), E);
             if (pair) {
               const C a2 = cscale(cadd(xs2, cscale(k2v, dt6)), E2);
-              if (wr) *rp.mir(a.acc, m) = a2;
+              if (wr) *rp.mir(acc, m) = a2;
               o2 = cscale(cadd(xs2, cscale(k2v, dt2)), E);
             }
           } else if (s == 2 || s == 3) {
             C a1 = slot[2 * G];
             a1 = cadd(a1, cscale(k1v, dt3 * E));
-            if (wr) *rp.at(a.acc, m) = a1;
+            if (wr) *rp.at(acc, m) = a1;
             const C x1 = slot[0];
             if (s == 2) o1 = cadd(cscale(x1, E), cscale(k1v, dt2));   // th3 = E th + dt/2 k
             else        o1 = cadd(cscale(x1, E2), cscale(k1v, tdt * E));       // th4 = E^2 th + dt E k
             if (pair) {
               C a2 = slot[3 * G];
               a2 = cadd(a2, cscale(k2v, dt3 * E));
-              if (wr) *rp.mir(a.acc, m) = a2;
+              if (wr) *rp.mir(acc, m) = a2;
               const C x2 = slot[G];
               if (s == 2) o2 = cadd(cscale(x2, E), cscale(k2v, dt2));
               else        o2 = cadd(cscale(x2, E2), cscale(k2v, tdt * E));
@@ -766,15 +770,15 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
             o1 = cadd(slot[2 * G], cscale(k1v, dt6));
             if (pair) o2 = cadd(slot[3 * G], cscale(k2v, dt6));
             if (wr) {
-              *rp.at(a.th_out, m) = o1;
-              if (pair) *rp.mir(a.th_out, m) = o2;
+              *rp.at(th_out, m) = o1;
+              if (pair) *rp.mir(th_out, m) = o2;
             }
           }
           if (FLAT && !act) o1 = o2 = mkc<C>(0, 0);
           if (s < 4 && wr) {
-            if (a.stage_write == SW_FULL || (a.stage_write == SW_RING && ring)) {
-              *rp.at(a.st_out, m) = o1;
-              if (pair) *rp.mir(a.st_out, m) = o2;
+            if (stage_write == SW_FULL || (stage_write == SW_RING && ring)) {
+              *rp.at(st_out, m) = o1;
+              if (pair) *rp.mir(st_out, m) = o2;
             }
           }
           bad |= !(cfinite(o1) && cfinite(o2));
@@ -787,16 +791,16 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
       if (m + DEPTH < R && (tail || in_band(m + DEPTH))) issue(m + DEPTH);
       if constexpr (DEPTH < R) cp_async_commit();  // (empty groups keep the in-order accounting)
     }
-    if (a.tl && tile_tail && a.do_p1 && rmode == RM_STAGE) {
+    if (tl && tile_tail && do_p1 && rmode == RM_STAGE) {
       // flags of theta_{s+1}'s rows: after the last stage those of the next
       // step; before it a row stays with every mode once it holds any (its
       // source or extra term put some there)
-      if (s == 4 && !a.extra) {
+      if (s == 4 && !extra) {
         const int any = __syncthreads_or(out_nz);
-        if (valid && j == 0) a.tl[p] = any ? 1 : 0;
+        if (valid && j == 0) tl[p] = any ? 1 : 0;
         skip_p1 = !any && tile_out;
       } else if (tail && valid && j == 0) {
-        a.tl[p] = 1;
+        tl[p] = 1;
       }
     }
   }
@@ -809,7 +813,7 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   if constexpr (NFX == 0 || ri_rmode(RI) == RM_RHS || ri_rmode(RI) == RM_SPEC) {
     return;
   } else {
-  if (!a.do_p1 || skip_p1) return;
+  if (!do_p1 || skip_p1) return;
 
   // Rows 0 and N/2 pair with themselves: e2 = (p, N - iy) is owned by another
   // thread of the group, so its new value is exchanged through shared memory
@@ -882,10 +886,10 @@ __device__ __forceinline__ void row_body(const KP& kp, const RowArgs& a, int til
   if constexpr (nfx_park(NFX)) fields(ha_smem);
   else fields(ha_reg);
   if constexpr (N <= R) __syncthreads();  // warp_out; longer transforms hold barriers
-  if (rmode == RM_P1 && a.tl && !tile_out && valid && j == 0) {
+  if (rmode == RM_P1 && tl && !tile_out && valid && j == 0) {
     bool any = false;
     for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) any |= warp_out[w];
-    a.tl[p] = any ? 1 : 0;
+    tl[p] = any ? 1 : 0;
   }
   }
 }
@@ -932,7 +936,8 @@ struct ColArgs {
   int herm_ord[4];          // ordinals of (0,0),(N/2,0),(0,N/2),(N/2,N/2) or -1
   double* ring_scale_out;   // [4]
   const unsigned char* tl;  // out-of-band flags of xh's rows: rows beyond pmax with flag 0 are zero and
-  const unsigned char* tl2; // unwritten (null: every row is written); of xh2's rows
+  const unsigned char* tl2; // unwritten (null: every row is written); of xh2's rows (null where tl is not:
+                            // every row of xh2 is written)
   int np;                   // column pairs per CTA (0: the compiled maximum NP)
   int tma;                  // 1: the half columns of xh arrive as TMA tiles through the
                             // kernel's tensor map (fields 0.. of the map = xh + f (N/2+1) N)
@@ -1086,14 +1091,13 @@ __device__ void ring_reduce(const KP& kp, const ColArgs& a);
 // Column pass.  NBUF = 4: all four fields of the column pairs are fetched at
 // once (round-2 copies land while round 1 computes); NBUF = 2: two rounds of
 // two fields (large N in float64, where four buffers do not fit).
-// CMX >= 0: an instance compiled for that column mode alone (the other
-// modes' branches fold away); -1: every mode, chosen by a.cmode at run time.
+// CMX: the column mode (the other modes' branches fold away).
 //
 // tm (non-null only from N = kColTmaMinN on, never in CM_SCALV): the field
 // stack xh as a tensor map; the half columns then arrive as TMA tiles (a
 // commit group's tiles complete on mbarrier colbar[g], one phase per group),
 // and a wait that runs out sets kStatusTmaTimeout in kp.status.
-template <typename T, int LOG2N, int R, int NP, int NBUF, int CMX = -1>
+template <typename T, int LOG2N, int R, int NP, int NBUF, int CMX>
 __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int tile, int ntiles,
                                          const CUtensorMap* tm = nullptr) {
   using C = typename Cplx<T>::type;
@@ -1103,8 +1107,8 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
   constexpr int SZ = ColBuf<N, R>::SZ;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C* smem = reinterpret_cast<C*>(smem_raw);
-  const int cmode = CMX >= 0 ? CMX : a.cmode;
-  if ((CMX < 0 || CMX == CM_THETA) && a.ring_cta && tile == ntiles - 1) {
+  constexpr int cmode = CMX;
+  if (CMX == CM_THETA && a.ring_cta && tile == ntiles - 1) {
     ring_reduce<T, LOG2N>(kp, a);
     return;
   }
@@ -1266,11 +1270,11 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
     }
     if (a.tl) {
       bool live = live_rows(a.tl);
-      if (cmode == CM_SCALV) live |= live_rows(a.tl2);
+      if (cmode == CM_SCALV) live = live || !a.tl2 || live_rows(a.tl2);
       if (__syncthreads_or(live)) {
         tl = a.tl;
         tl2 = cmode == CM_SCALV ? a.tl2 : a.tl;
-        if (!BYROW) dead = __syncthreads_or(any_row(tl, false) || any_row(tl2, false));
+        if (!BYROW) dead = __syncthreads_or(any_row(tl, false) || (tl2 && any_row(tl2, false)));
         fetch_rest(xh + fa0 * fstride, 0, fa0, &colbar[0]);
         fetch_rest(xb + fb0s * fstride, 1, fb0s, &colbar[0]);
         if (two) {
@@ -1300,7 +1304,7 @@ __device__ __forceinline__ void col_body(const KP& kp, const ColArgs& a, int til
         zero_rows(1, 4, tl);
       } else {
         zero_rows(2, 2, tl);
-        zero_rows(2, 2, tl2, 1);
+        if (tl2) zero_rows(2, 2, tl2, 1);
       }
       __syncthreads();
     }
@@ -1489,14 +1493,14 @@ __device__ void ring_reduce(const KP& kp, const ColArgs& a) {
 
 namespace sqg {
 // ---- kernels: one plan, or a batch of members (member = blockIdx.y) ----
-template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI = RI_ANY>
+template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI>
 __global__ void __launch_bounds__(RPC * ((1 << LOG2N) / R), row_min_blocks<T, R, NFX>(RPC * ((1 << LOG2N) / R)))
 k_row(KP kp, RowArgs a) {
   pdl_wait();
   row_body<T, LOG2N, R, RPC, DEPTH, NFX, RI>(kp, a, blockIdx.x);
 }
 
-template <typename T, int LOG2N, int R, int NP, int NBUF, int CMX = -1>
+template <typename T, int LOG2N, int R, int NP, int NBUF, int CMX>
 __global__ void __launch_bounds__(NP * ((1 << LOG2N) / R), min_blocks_r<T, R>(NP * ((1 << LOG2N) / R)))
 k_col(KP kp, ColArgs a, const __grid_constant__ CUtensorMap tm) {
   pdl_wait();
@@ -1505,23 +1509,23 @@ k_col(KP kp, ColArgs a, const __grid_constant__ CUtensorMap tm) {
 
 // Batched forms: the member's parameters come from device arrays; members
 // with no work in this pass have a null xh pointer and return at once.
-template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX>
+template <typename T, int LOG2N, int R, int RPC, int DEPTH, int NFX, int RI>
 __global__ void __launch_bounds__(RPC * ((1 << LOG2N) / R), row_min_blocks<T, R, NFX>(RPC * ((1 << LOG2N) / R)))
 k_row_batch(const KP* __restrict__ kps, const RowArgs* __restrict__ as) {
   pdl_wait();
   const KP& kp = kps[blockIdx.y];  // read in place (a local copy would be indexed dynamically)
   const RowArgs& a = as[blockIdx.y];
   if (a.xh == nullptr && a.rhs_out == nullptr) return;
-  row_body<T, LOG2N, R, RPC, DEPTH, NFX>(kp, a, blockIdx.x);
+  row_body<T, LOG2N, R, RPC, DEPTH, NFX, RI, true>(kp, a, blockIdx.x);
 }
 
-template <typename T, int LOG2N, int R, int NP, int NBUF>
+template <typename T, int LOG2N, int R, int NP, int NBUF, int CMX>
 __global__ void __launch_bounds__(NP * ((1 << LOG2N) / R), min_blocks_r<T, R>(NP * ((1 << LOG2N) / R)))
 k_col_batch(const KP* __restrict__ kps, const ColArgs* __restrict__ as) {
   pdl_wait();
   const KP& kp = kps[blockIdx.y];
   const ColArgs& a = as[blockIdx.y];
   if (a.xh == nullptr) return;
-  col_body<T, LOG2N, R, NP, NBUF>(kp, a, blockIdx.x, gridDim.x);
+  col_body<T, LOG2N, R, NP, NBUF, CMX>(kp, a, blockIdx.x, gridDim.x);
 }
 }  // namespace sqg

@@ -152,8 +152,12 @@ template <typename T, int L>
 cudaError_t launch_col_t(const KP& kp, const ColArgs& a, cudaStream_t st, bool ring_only, const CUtensorMap* tm);
 template <typename T, int L> cudaError_t shape_max_t(int* rpc, int* np);
 template <typename T, int L> cudaError_t set_attrs_t();
-template <typename T, int L> cudaError_t launch_row_batch_t(const KP* kps, const RowArgs* as, int members, cudaStream_t st);
-template <typename T, int L> cudaError_t launch_col_batch_t(const KP* kps, const ColArgs* as, int members, cudaStream_t st);
+// (batches: ri one of RI_THETA_P1, RI_SCAL_P1, RI_THETA_STAGE, RI_SCAL_STAGE; cm
+// CM_THETA, CM_SCAL or CM_VEL)
+template <typename T, int L>
+cudaError_t launch_row_batch_t(const KP* kps, const RowArgs* as, int members, int ri, cudaStream_t st);
+template <typename T, int L>
+cudaError_t launch_col_batch_t(const KP* kps, const ColArgs* as, int members, int cm, cudaStream_t st);
 template <typename T, int L> cudaError_t set_batch_attrs_t();
 
 // ---- multi-size ensemble passes ----
@@ -339,28 +343,60 @@ cudaError_t set_attrs_t() {
   return e;
 }
 
-template <typename T, int L>
-cudaError_t launch_row_batch_t(const KP* kps, const RowArgs* as, int members, cudaStream_t st) {
+template <typename T, int L, int RI>
+cudaError_t launch_row_batch_i(const KP* kps, const RowArgs* as, int members, cudaStream_t st) {
   constexpr int N = 1 << L, RPC = rows_per_cta<T, L>();
   dim3 grid((N / 2 + 1 + RPC - 1) / RPC, members);
-  return launch_pdl(k_row_batch<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>()>, grid,
+  return launch_pdl(k_row_batch<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>(), RI>, grid,
                     dim3(RPC * row_group<T, L>()), row_smem<T, L>(), st, kps, as);
 }
 template <typename T, int L>
-cudaError_t launch_col_batch_t(const KP* kps, const ColArgs* as, int members, cudaStream_t st) {
+cudaError_t launch_row_batch_t(const KP* kps, const RowArgs* as, int members, int ri, cudaStream_t st) {
+  switch (ri) {
+    case RI_THETA_P1: return launch_row_batch_i<T, L, RI_THETA_P1>(kps, as, members, st);
+    case RI_SCAL_P1: return launch_row_batch_i<T, L, RI_SCAL_P1>(kps, as, members, st);
+    case RI_THETA_STAGE: return launch_row_batch_i<T, L, RI_THETA_STAGE>(kps, as, members, st);
+    case RI_SCAL_STAGE: return launch_row_batch_i<T, L, RI_SCAL_STAGE>(kps, as, members, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template <typename T, int L, int CMX>
+cudaError_t launch_col_batch_i(const KP* kps, const ColArgs* as, int members, cudaStream_t st) {
   constexpr int N = 1 << L, NP = pairs_per_cta<T, L>();
   dim3 grid(N / (2 * NP), members);
-  return launch_pdl(k_col_batch<T, L, col_radix<T, L>(), NP, col_nbuf<T, L>()>, grid,
+  return launch_pdl(k_col_batch<T, L, col_radix<T, L>(), NP, col_nbuf<T, L>(), CMX>, grid,
                     dim3(NP * col_group<T, L>()), col_smem<T, L>(), st, kps, as);
 }
 template <typename T, int L>
-cudaError_t set_batch_attrs_t() {
-  constexpr int RPC = rows_per_cta<T, L>(), NP = pairs_per_cta<T, L>();
-  cudaError_t e = cudaFuncSetAttribute(k_row_batch<T, L, row_radix<T, L>(), RPC, row_depth<T, L>(), row_nfx<T, L>()>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T, L>());
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_col_batch<T, L, col_radix<T, L>(), NP, col_nbuf<T, L>()>,
+cudaError_t launch_col_batch_t(const KP* kps, const ColArgs* as, int members, int cm, cudaStream_t st) {
+  switch (cm) {
+    case CM_THETA: return launch_col_batch_i<T, L, CM_THETA>(kps, as, members, st);
+    case CM_SCAL: return launch_col_batch_i<T, L, CM_SCAL>(kps, as, members, st);
+    case CM_VEL: return launch_col_batch_i<T, L, CM_VEL>(kps, as, members, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template <typename T, int L, int RI>
+cudaError_t set_row_batch_attrs_i() {
+  return cudaFuncSetAttribute(
+      k_row_batch<T, L, row_radix<T, L>(), rows_per_cta<T, L>(), row_depth<T, L>(), row_nfx<T, L>(), RI>,
+      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem<T, L>());
+}
+template <typename T, int L, int CMX>
+cudaError_t set_col_batch_attrs_i() {
+  return cudaFuncSetAttribute(k_col_batch<T, L, col_radix<T, L>(), pairs_per_cta<T, L>(), col_nbuf<T, L>(), CMX>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem<T, L>());
+}
+template <typename T, int L>
+cudaError_t set_batch_attrs_t() {
+  cudaError_t e = set_row_batch_attrs_i<T, L, RI_THETA_P1>();
+  if (e == cudaSuccess) e = set_row_batch_attrs_i<T, L, RI_SCAL_P1>();
+  if (e == cudaSuccess) e = set_row_batch_attrs_i<T, L, RI_THETA_STAGE>();
+  if (e == cudaSuccess) e = set_row_batch_attrs_i<T, L, RI_SCAL_STAGE>();
+  if (e == cudaSuccess) e = set_col_batch_attrs_i<T, L, CM_THETA>();
+  if (e == cudaSuccess) e = set_col_batch_attrs_i<T, L, CM_SCAL>();
+  if (e == cudaSuccess) e = set_col_batch_attrs_i<T, L, CM_VEL>();
+  return e;
 }
 
 // Explicit instantiation of every launch function for one (T, log2 N).
@@ -369,8 +405,8 @@ cudaError_t set_batch_attrs_t() {
   template cudaError_t launch_col_t<T, L>(const KP&, const ColArgs&, cudaStream_t, bool, const CUtensorMap*); \
   template cudaError_t shape_max_t<T, L>(int*, int*);                                                      \
   template cudaError_t set_attrs_t<T, L>();                                                                \
-  template cudaError_t launch_row_batch_t<T, L>(const KP*, const RowArgs*, int, cudaStream_t);             \
-  template cudaError_t launch_col_batch_t<T, L>(const KP*, const ColArgs*, int, cudaStream_t);             \
+  template cudaError_t launch_row_batch_t<T, L>(const KP*, const RowArgs*, int, int, cudaStream_t);        \
+  template cudaError_t launch_col_batch_t<T, L>(const KP*, const ColArgs*, int, int, cudaStream_t);        \
   template cudaError_t set_batch_attrs_t<T, L>();
 #endif
 
