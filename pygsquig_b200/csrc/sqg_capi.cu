@@ -1499,15 +1499,16 @@ cudaError_t bcol(sqg_batch* b, const KP* kps, const ColArgs* as, int m, int cm, 
                                    : launch_col_batch_p<float>(b->log2N, kps, as, m, cm, st);
 }
 
-// Whether theta's (the scalars') passes of an ensemble's size class keep flags of
-// their rows.  They pay where rows are skipped and cost where none is, the less
-// the longer a row; a theta's rows outside the band are soon emptied by
-// hyperviscosity, a scalar's diffusion leaves round-off there for thousands of
-// steps.  Three steps, every row live (after the second slash: none outside the band),
-// with both flags and without: N = 64 x 48 FP32 320 and 293 us / 283 and 290;
-// 128 x 48 FP64 1251 and 1181 / 921 and 1199; 256 x 24 FP64 2458 and 2313 / 1867
-// and 2309; 512 x 12 FP32 1994 and 2162 / 1639 and 2153.
-bool batch_flags(int N, bool theta) { return N >= (theta ? 128 : 256); }
+// Whether theta's (the scalars') passes of a size class of M members keep flags
+// of their rows.  They pay where rows are skipped and cost where none is, the less
+// the longer a row and the fuller the chip; a theta's rows outside the band are
+// soon emptied by hyperviscosity, a scalar's diffusion leaves round-off there for
+// thousands of steps.  Three steps of theta and scalars, every row live (after the
+// second slash: none outside the band), with flags and without: N = 64 x 48 FP32
+// 320 and 293 us / 283 and 290; 128 x 48 FP64 1251 and 1181 / 921 and 1199 (theta's
+// flags alone 1208 / 1051); 128 x 1 FP64 369 and 348 / 339 and 351; 256 x 24 FP64
+// 2458 and 2313 / 1867 and 2309; 512 x 12 FP32 1994 and 2162 / 1639 and 2153.
+bool batch_flags(int N, int M, bool theta) { return N >= 256 || (theta && N == 128 && M >= 16); }
 
 // Builds and uploads every member's pass arguments for time step dt.
 int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
@@ -1538,7 +1539,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     a.th_n = b->mem[i].theta;
     a.th_out = b->mem[i].theta;
     a.do_p1 = 1;
-    a.tl = batch_flags(b->N, true) ? mb + b->m_tl : nullptr;
+    a.tl = batch_flags(b->N, b->M, true) ? mb + b->m_tl : nullptr;
     p1[i] = a;
     p1[i].rmode = RM_P1;
     for (int s = 1; s <= 4; ++s) {
@@ -1579,7 +1580,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     a.th_out = b->mem[i].scalars[q];
     a.kappa = b->mem[i].kappa[q];
     a.do_p1 = 1;
-    a.tl = batch_flags(b->N, false) ? sb + b->s_tl : nullptr;
+    a.tl = batch_flags(b->N, b->M, false) ? sb + b->s_tl : nullptr;
     sp1[k] = a;
     sp1[k].rmode = RM_P1;
     const bool sexp = b->d.scheme == SQG_EXPLICIT_RK4 && a.kappa != 0.0;
@@ -1606,7 +1607,7 @@ int batch_upload_args(sqg_batch* b, double dt, cudaStream_t st) {
     cv.cmode = CM_SCALV;
     cv.xh = mb + b->m_xh;
     cv.xh2 = a.xh;
-    cv.tl = batch_flags(b->N, true) ? mb + b->m_tl : nullptr;
+    cv.tl = batch_flags(b->N, b->M, true) ? mb + b->m_tl : nullptr;
     cv.tl2 = a.tl;
     cv.out0 = q == 0 ? mb + b->m_uv : nullptr;
     scolv[k] = cv;
