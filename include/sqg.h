@@ -165,7 +165,7 @@ int sqg_multistep(sqg_plan* plan, void* theta_hat, int32_t n_steps, double dt,
  *   sqg_stage_begin(theta_in); then for s = 1..4:
  *     extra_s = f(theta_s)   (theta_s = theta_in for s = 1, else SQG_BUF_STAGE)
  *     sqg_stage(s, extra_s)
- * After stage 4 theta_out holds the new state.  extra may be NULL. */
+ * After stage 4 theta_out holds the new state.  extra may be NULL at any stage. */
 int sqg_stage_begin(sqg_plan* plan, const void* theta_in, void* stream);
 int sqg_stage(sqg_plan* plan, int32_t stage, const void* theta_in, void* theta_out,
               double dt, const void* extra_rhs, const double* ring_phases, void* stream);
@@ -278,7 +278,9 @@ int sqg_ensemble_multistep(sqg_ensemble* ensemble, int32_t n_steps, double dt, i
 int sqg_ensemble_last_launch_count(const sqg_ensemble* ensemble, int64_t* launches);
 int sqg_ensemble_destroy(sqg_ensemble* ensemble);
 
-/* Reads and clears the sticky status flags (bit 0: non-finite value seen;
+/* Reads and clears the sticky status flags (bit 0: non-finite value seen in a
+ * new field or stage; an advective term that overflows at none but modes the
+ * dealiasing mask discards is discarded there and not seen;
  * bit 1: a column pass's TMA tile copies did not complete within its bounded
  * wait, so its results are not valid).  Synchronises the stream. */
 int sqg_check_status(sqg_plan* plan, uint32_t* flags, void* stream);

@@ -44,8 +44,9 @@ int closure_wgrad64(int32_t B, int32_t H, int32_t W, const void* act_pad, const 
                     int32_t nparts, float* dw, uint32_t* err, void* stream);
 
 /* CUDA-core kernels of the 1-channel layers and the training step
- * (W a multiple of 32, H >= 2; a warp owns 32 pixels of a row, a lane a
- * channel pair).
+ * (W a multiple of 32, H >= 2; a warp owns 32 pixels of a row).  Tensors of
+ * 64 channels start on 16 bytes, those of conv_out_dgrad, small_grad and the
+ * input of conv_out on 4.
  * conv_in:  z = conv3x3(in_scale x; w[9][64]) + bias (1 -> 64); z BF16
  *           [B][H][W][64], a_pad = gelu(z) BF16 halo'd.  x: FP32 [B][H][W].
  * conv_out: y = out_scale (conv3x3(a; w[9][64]) + bias[0]) (64 -> 1), y FP32

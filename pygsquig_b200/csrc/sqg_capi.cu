@@ -373,7 +373,7 @@ cudaError_t launch_col(sqg_plan* pl, const KP& kp, const ColArgs& a, cudaStream_
 // on small grids: a single small field is one wave of blocks bound by latency,
 // where the flags' load costs more than the skipped rows give (N = 256 FP64 step
 // 59.6 us without, 73 us with them; N = 512 FP32 58 us without, 58 or, with every
-// row flagged, 65 with them; FP64 there 85 without, 76 or 83 with them).
+// row flagged, 65 with them; FP64 there 78 without, 76 or 82 with them).
 unsigned char* band_flags(const sqg_plan* pl, size_t off) {
   const int min_n = pl->d.precision == SQG_F64 ? 512 : 1024;
   return pl->band_ok && off && pl->N >= min_n ? pl->ws + off : nullptr;

@@ -302,9 +302,10 @@ __device__ __forceinline__ void fft_elems(E (&v)[NE][R], E* sbuf, int bstride, i
   // pass's root is loaded one pass ahead so the load's latency (the table is
   // often not L1-resident next to large shared-memory buffers) overlaps the
   // butterflies and exchange of the pass before.
-  // (TW2: w and w^3 from the table instead of w alone: powers of w carry its
-  // rounding r-fold, and the radix-8 row pass that serves N = 2048 instead of a
-  // radix-4 one is to be no further from exact: at w, w^3 the squared errors of
+  // (TW2, every radix-8 transform of N = 2048 -- the row pass of both precisions
+  // and the column pass in double: w and w^3 from the table instead of w alone.
+  // Powers of w carry its rounding r-fold, and the row pass there, radix 8 instead
+  // of radix 4, is to be no further from exact: at w, w^3 the squared errors of
   // its twiddles sum to 12 units over its passes, to 17.5 in radix 4, to 52 from
   // w alone.)
   constexpr bool TW2 = fft_tw2<T, LOG2N, R>();

@@ -47,10 +47,13 @@ struct RowTab {
 // The band of a field: the disk p <= pmax, p^2 + m_y^2 <= s2 (mode numbers) that
 // holds the dealiasing mask.  Modes outside it -- half of a spectrum's rows
 // times columns, a third of the rows p = 0..N/2 entirely -- get no advective
-// tendency, so a spectrum that is zero there stays zero through a step, and a
-// run's is: what an initial field holds there decays by hyperviscosity alone,
-// and a spectrum interpolated or restarted from a band-limited one never held
-// any.  The input pass of a step sets one byte per row pair, tl[p] = 1 when the
+// tendency, so a spectrum that is zero there stays zero through a step.  A
+// spectrum interpolated or restarted from a band-limited one is; what a field
+// from physical space holds there is round-off that only its linear operator
+// removes: hyperviscosity that empties it within some tens of steps for theta of
+// a forced run, a scalar's diffusion not for thousands (and in single precision a
+// factor near one leaves its last subnormal units for good), so such fields keep
+// every mode.  The input pass of a step sets one byte per row pair, tl[p] = 1 when the
 // pair holds a non-zero mode outside the band.  With tl[p] = 0 the stage passes
 // load, update and store the band's modes only, and a row beyond pmax costs
 // its block one byte: no transforms, no half-spectrum rows (the column pass
